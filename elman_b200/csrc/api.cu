@@ -208,6 +208,13 @@ static bool dense_tc_ok(int dtype, int T, int B, int d, int bwd) {
   return use_tc(dtype) && rec_tc_supported(T, B, d, bwd);
 }
 
+// The recurrence with W in registers, unless the caller asks for the smallest footprint and the
+// TMEM kernel has a plan for that.
+static bool reg_ok(int dtype, int T, int B, int d, int compact) {
+  return use_tc(dtype) && rec_reg_supported(T, B, d) &&
+         !(compact && rec_tc_supported(T, B, d, 0) && rec_tc_supported(T, B, d, 1));
+}
+
 // ---------------------------------------------------------------------------
 // E1
 // ---------------------------------------------------------------------------
@@ -226,7 +233,7 @@ static size_t carve_e1_bwd(int dtype, int T, int B, int d, void* ws, E1BwdWs* o)
   size_t es = esize(dtype);
   o->Wt = c.take((size_t)d * d * es);
   o->dv = c.take((size_t)(T + 1) * B * d * es);  // slot T: zero "gradient from the future"
-  o->db = (float*)c.take((size_t)REC_MAX_REPLICAS * d * sizeof(float));
+  o->db = (float*)c.take((size_t)REC_MAX_DB_ROWS * d * sizeof(float));
   size_t sb = rec_sync_bytes() > rec_tc_sync_bytes() ? rec_sync_bytes() : rec_tc_sync_bytes();
   o->sync = (int*)c.take(sb);
   o->WxT = nullptr;  // the GEMMs read transposed operands in place
@@ -241,6 +248,10 @@ static int run_rec_fwd(int dtype, int T, int B, int d, const void* W, const void
   PhaseTimer timer(0, st);
   RecFwdArgs a{T, B, d, W, pre, g, h, y, v, sync};
   a.compact = compact;
+  if (reg_ok(dtype, T, B, d, compact)) {
+    const int rc = rec_fwd_reg(a, st);
+    if (rc != ELMAN_ERR_UNSUPPORTED) return rc;   // an unaligned operand: nothing was launched
+  }
   if (dense_tc_ok(dtype, T, B, d, 0)) {
     // a plan that was co-resident when it was made may not be at launch time (another
     // context holds SMs): nothing was launched then, and the CUDA-core kernel takes over
@@ -266,6 +277,10 @@ static int run_rec_bwd(int dtype, int T, int B, int d, const void* Wt, const voi
   PhaseTimer timer(1, st);
   RecBwdArgs a{T, B, d, Wt, h, v, g, dy, dv, dg, db, sync};
   a.compact = compact;
+  if (reg_ok(dtype, T, B, d, compact)) {
+    const int rc = rec_bwd_reg(a, st);
+    if (rc != ELMAN_ERR_UNSUPPORTED) return rc;
+  }
   if (dense_tc_ok(dtype, T, B, d, 1)) {
     const int rc = rec_bwd_tc(a, st);
     if (rc != ELMAN_ERR_UNSUPPORTED) return rc;   // see run_rec_fwd
@@ -307,6 +322,7 @@ int elman_b200_set_option(const char* name, long value) {
   else if (!strcmp(name, "time_kernels")) o.time_kernels = value;
   else if (!strcmp(name, "rec_trace")) o.rec_trace = value;
   else if (!strcmp(name, "rec_mma_warps")) o.rec_mma_warps = value;
+  else if (!strcmp(name, "rec_reg")) o.rec_reg = value;
   else if (!strcmp(name, "rec_direct_publish")) o.rec_direct_publish = value;
   else if (!strcmp(name, "rec_w_tmem")) o.rec_w_tmem = value;
   else if (!strcmp(name, "rec_large_batch")) o.rec_large_batch = value;
@@ -330,6 +346,7 @@ long elman_b200_get_option(const char* name) {
   if (!strcmp(name, "time_kernels")) return o.time_kernels;
   if (!strcmp(name, "rec_trace")) return o.rec_trace;
   if (!strcmp(name, "rec_mma_warps")) return o.rec_mma_warps;
+  if (!strcmp(name, "rec_reg")) return o.rec_reg;
   if (!strcmp(name, "rec_direct_publish")) return o.rec_direct_publish;
   if (!strcmp(name, "rec_w_tmem")) return o.rec_w_tmem;
   if (!strcmp(name, "rec_large_batch")) return o.rec_large_batch;
@@ -361,8 +378,10 @@ long elman_b200_tc_launch_count(void) { return g_tc_launches.load(); }
 
 int elman_b200_recurrence_blocks(int dtype, int flags, int T, int B, int d) {
   if (T <= 0 || B <= 0 || d <= 0) return 0;
-  return dense_tc_ok(dtype, T, B, d, 0) && dense_tc_ok(dtype, T, B, d, 1) ? rec_tc_blocks(T, B, d, (flags & ELMAN_FLAG_COMPACT) ? 1 : 0)
-                                     : 0;
+  const int compact = (flags & ELMAN_FLAG_COMPACT) ? 1 : 0;
+  if (reg_ok(dtype, T, B, d, compact)) return rec_reg_blocks(B, d);
+  return dense_tc_ok(dtype, T, B, d, 0) && dense_tc_ok(dtype, T, B, d, 1)
+             ? rec_tc_blocks(T, B, d, compact) : 0;
 }
 
 // ------------------------------- E1 ----------------------------------------
@@ -579,7 +598,7 @@ static size_t carve_e0_bwd(int dtype, int T, int B, int d, void* ws, E0BwdWs* o)
   o->Wt = c.take((size_t)d * d * es);
   o->dv = c.take((size_t)(T + 1) * B * d * es);  // slot T: zero "gradient from the future"
   o->dg = c.take((size_t)T * B * d * es);
-  o->db = (float*)c.take((size_t)REC_MAX_REPLICAS * d * sizeof(float));
+  o->db = (float*)c.take((size_t)REC_MAX_DB_ROWS * d * sizeof(float));
   o->cs = (float*)c.take(column_sum_scratch_bytes(d));
   size_t sb = rec_sync_bytes() > rec_tc_sync_bytes() ? rec_sync_bytes() : rec_tc_sync_bytes();
   o->sync = (int*)c.take(sb);
@@ -1126,7 +1145,7 @@ struct E1RecWs { void* Wt; float* db; int* sync; };
 static size_t carve_e1_rec(int dtype, int d, void* ws, E1RecWs* o) {
   Carver c(ws);
   o->Wt = c.take((size_t)d * d * esize(dtype));
-  o->db = (float*)c.take((size_t)REC_MAX_REPLICAS * d * sizeof(float));
+  o->db = (float*)c.take((size_t)REC_MAX_DB_ROWS * d * sizeof(float));
   size_t sb = rec_sync_bytes() > rec_tc_sync_bytes() ? rec_sync_bytes() : rec_tc_sync_bytes();
   o->sync = (int*)c.take(sb);
   return c.total();
@@ -1271,7 +1290,7 @@ static size_t carve_hx_bwd(int dtype, int T, int B, int d, void* ws, HxBwdWs* o)
   const size_t es = esize(dtype), TBd = (size_t)T * B * d * es;
   o->Wt = c.take((size_t)d * d * es);
   o->dv = c.take(TBd + (size_t)B * d * es);
-  o->db = (float*)c.take((size_t)REC_MAX_REPLICAS * d * sizeof(float));
+  o->db = (float*)c.take((size_t)REC_MAX_DB_ROWS * d * sizeof(float));
   size_t sb = rec_sync_bytes() > rec_tc_sync_bytes() ? rec_sync_bytes() : rec_tc_sync_bytes();
   o->sync = (int*)c.take(sb);
   o->splitk_bytes = splitk_scratch_bytes(dtype, d, d);

@@ -48,6 +48,7 @@ struct Options {
   long time_kernels = 0;
   long rec_trace = 0;
   long rec_mma_warps = 0;
+  long rec_reg = 0;            // 0 auto, 1 never: the recurrence with W in registers
   long rec_direct_publish = 0;
   long rec_w_tmem = 0;
   long gemm_persistent = 0;    // 0 auto, 1 never, 2 always: the persistent 128x256 GEMM kernel
@@ -241,14 +242,28 @@ int lowrank_bwd_generic(int dtype, const LowRankBwdArgs& a, cudaStream_t stream)
 
 // Dense recurrence, bf16, tcgen05 + TMA persistent cluster kernel.
 // Batch replicas of a recurrence grid (throughput plan); the backward kernel writes one row of
-// bias-gradient sums per replica, so callers give its `db` REC_MAX_REPLICAS * d floats.
+// bias-gradient sums per replica, so callers give its `db` REC_MAX_DB_ROWS * d floats.
 constexpr int REC_MAX_REPLICAS = 4;
+// Rows of bias-gradient sums (one per replica or batch group) a recurrence may write before they
+// are folded into the first.
+constexpr int REC_MAX_DB_ROWS = 16;
+int fold_db_rows(float* db, int d, int rows, cudaStream_t stream);
 bool rec_tc_supported(int T, int B, int d, int bwd);   // per direction: the plans differ
 // resident thread blocks of one launch (compact: smallest-footprint plan), 0 if unsupported
 int rec_tc_blocks(int T, int B, int d, int compact);
 size_t rec_tc_sync_bytes();
 int rec_fwd_tc(const RecFwdArgs& a, cudaStream_t stream);
 int rec_bwd_tc(const RecBwdArgs& a, cudaStream_t stream);
+
+// Dense recurrence, bf16, W in registers (rec_reg.cuh): up to RR_MAX_BATCH rows, d % 8 == 0,
+// d <= 2048.  Launches that may overlap others have d >= RR_MIN_CONCURRENT_D.
+constexpr int RR_MAX_BATCH = 64;
+constexpr int RR_MIN_CONCURRENT_D = 128;
+bool rec_reg_supported(int T, int B, int d);
+int rec_reg_blocks(int B, int d);
+int rec_fwd_reg(const RecFwdArgs& a, cudaStream_t stream);
+int rec_bwd_reg(const RecBwdArgs& a, cudaStream_t stream);
+
 // Copies the cycle stamps of the last traced launch (option rec_trace) to the host.
 int rec_tc_copy_trace(long long* dst, int max_entries);
 void set_last_trace(long long* device_buffer);   // the buffer the next copy reads

@@ -1,0 +1,171 @@
+// Plans and launches of the register-resident recurrence (rec_reg.cuh).
+#include <map>
+#include <mutex>
+#include <tuple>
+
+#include "rec_reg_table.cuh"
+
+namespace elman {
+
+namespace {
+
+struct RecRegPlan {
+  int mt, kb, nt;
+  int groups, cpg;
+  bool ok;
+};
+
+int device_sms() {
+  static int sms[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return 0; }
+  if (sms[dev] == 0 &&
+      cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    cudaGetLastError();
+  return sms[dev];
+}
+
+// MB of state that one look of all CTAs together reads.
+double rr_look_mb(int B, int d, int cpg) { return (double)B * d * 2 * cpg / 1e6; }
+
+// Cycles from a step's barrier to the first look at the next state.  What a warp with outputs has
+// to do until then takes about 700; a look that comes too early costs its own round trip and the
+// L2 bandwidth that the other CTAs' looks and stores need (d = 1280, B = 32, 108 CTAs: 1.60 us per
+// step without the wait, 1.38 with 800 cycles; B = 3, 80 CTAs: 1.25 and 0.98 with 600).
+int rr_hold(int B, int d, int cpg) {
+  const double mb = rr_look_mb(B, d, cpg);
+  const int cycles = mb < 0.5 ? 450 : (int)(560 + 110 * mb);
+  return cycles > 1000 ? 1000 : cycles;
+}
+
+// Groups of 8 or 16 rows, 16 to 64 rows of W per CTA.  Time of a step in ns, fitted to all plans of
+// ten shapes (B 3 to 64, d 256 to 2048; 5 % mean error): 680 for the hand-off through L2 and what
+// follows the barrier, 11 per KB of state a CTA reads, 18 per m-tile, n-tile and K block (the
+// tensor pipe does an m16n8k16 in 2 cycles per SM), 36 per m-tile and n-tile of partial sums, 43
+// per MB that all CTAs read together.  Measured, us per step forward / backward:
+//
+//    B    d   TMEM kernel   NT MT CTAs   this kernel
+//    3  1280   3.96 3.86     1  1   80   0.98 0.99
+//   32  1280   4.27 4.39     1  4   80   1.47 1.54     (MT = 3, 108 CTAs: 1.38 1.43)
+//   48   768   4.70 4.72     1  3   96   1.19 1.27
+//   64  1280   5.37 5.49     2  3  108   2.04 2.12
+//   32  2048   4.81 4.85     2  2  128   2.21 2.24
+//   37   952    55   40      1  4   75   1.33 1.41     (no TMEM plan: CUDA cores)
+//
+// Among plans within 8 % of the best estimate the one with the fewest CTAs is taken: the SMs it
+// leaves alone serve other streams.
+RecRegPlan pick_rec_reg_plan(int B, int d) {
+  RecRegPlan best{};
+  best.ok = false;
+  const int kb = ((d + 31) / 32 + RR_WARPS - 1) / RR_WARPS;
+  if (B < 1 || B > RR_MAX_BATCH || d < 8 || (d & 7) != 0 || kb > RR_MAX_KB) return best;
+  const int sms = device_sms();
+  double best_cost = 0;
+  for (int pass = 0; pass < 2; ++pass) {
+    int best_ctas = 0;
+    for (int nt = 1; nt <= RR_MAX_NT; ++nt)
+      for (int mt = 1; mt <= RR_MAX_MT; ++mt) {
+        if (mt * kb > RR_MAX_W) continue;
+        const int groups = (B + 8 * nt - 1) / (8 * nt), cpg = (d + 16 * mt - 1) / (16 * mt);
+        const int ctas = groups * cpg;
+        if (ctas > sms || groups > REC_MAX_DB_ROWS) continue;
+        const double in_kb = d * 2.0 * (B < 8 * nt ? B : 8 * nt) / 1024;
+        const double cost = 680 + 11 * in_kb + 18.0 * mt * nt * kb + 36.0 * mt * nt +
+                            43 * rr_look_mb(B, d, cpg);
+        if (pass == 0) {
+          if (best_cost == 0 || cost < best_cost) best_cost = cost;
+        } else if (cost <= 1.08 * best_cost && (best_ctas == 0 || ctas < best_ctas)) {
+          best_ctas = ctas;
+          best.mt = mt; best.kb = kb; best.nt = nt; best.groups = groups; best.cpg = cpg;
+          best.ok = true;
+        }
+      }
+  }
+  return best;
+}
+
+// Options that select a plan of the TMEM kernel select that kernel.
+bool rr_enabled() {
+  const Options& o = options();
+  return o.rec_reg != 1 && o.rec_ksplit == 0 && o.rec_groups == 0 && o.rec_mma_warps == 0 &&
+         o.rec_trace == 0;
+}
+
+int rr_launch(bool bwd, const RecRegPlan& pl, RecRegParams& p, int* sync, cudaStream_t stream) {
+  RecRegKernel kern = bwd ? rec_reg_bwd_kernel(pl.mt, pl.kb, pl.nt)
+                          : rec_reg_fwd_kernel(pl.mt, pl.kb, pl.nt);
+  // rows of W and of the state are read 16 bytes at a time, the rest in feature pairs
+  const uintptr_t wide = (uintptr_t)p.W | (uintptr_t)p.state;
+  const uintptr_t narrow = (uintptr_t)p.in0 | (uintptr_t)p.in1 | (uintptr_t)p.in2 | (uintptr_t)p.in3 |
+                           (uintptr_t)p.out0 | (uintptr_t)p.out1;
+  if (kern == nullptr || (wide & 15) != 0 || (narrow & 3) != 0) return ELMAN_ERR_UNSUPPORTED;
+  const size_t smem = rec_reg_smem(bwd, pl.mt, pl.nt);
+  if (smem > 48 * 1024)
+    ELMAN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  p.cpg = pl.cpg;
+  p.hold = rr_hold(p.B, p.d, pl.cpg);
+  p.abort_word = sync;
+  p.status = device_status_ptr();
+  p.spin_limit = options().spin_limit;
+  p.stall_step = (int)options().test_stall_step;
+  ELMAN_CUDA_CHECK(cudaMemsetAsync(sync, 0, 4, stream));
+  // every slot the kernel writes starts out as "not there yet"
+  const size_t slot = (size_t)p.B * p.d * sizeof(bf16);
+  ELMAN_CUDA_CHECK(cudaMemsetAsync((char*)p.state + (bwd ? 0 : slot), 0xFF, (size_t)p.T * slot, stream));
+  // CTAs wait for one another.  A cooperative launch is the runtime's guarantee that they are
+  // resident together; shapes under 128 features, which callers that overlap launches do not
+  // plan for (elman_b200_recurrence_blocks reports 0), ask for it.
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(pl.groups * pl.cpg);
+  cfg.blockDim = dim3(RR_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeCooperative;
+  attr.val.cooperative = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = p.d < RR_MIN_CONCURRENT_D ? 1 : 0;
+  ELMAN_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, (const RecRegParams)p));
+  count_launch(true);
+  return ELMAN_OK;
+}
+
+}  // namespace
+
+bool rec_reg_supported(int T, int B, int d) {
+  return T >= 1 && rr_enabled() && pick_rec_reg_plan(B, d).ok;
+}
+
+int rec_reg_blocks(int B, int d) {
+  const RecRegPlan pl = pick_rec_reg_plan(B, d);
+  return pl.ok && d >= RR_MIN_CONCURRENT_D ? pl.groups * pl.cpg : 0;
+}
+
+int rec_fwd_reg(const RecFwdArgs& a, cudaStream_t stream) {
+  const RecRegPlan pl = pick_rec_reg_plan(a.B, a.d);
+  if (!pl.ok) return ELMAN_ERR_UNSUPPORTED;
+  RecRegParams p{};
+  p.T = a.T; p.B = a.B; p.d = a.d;
+  p.W = (const bf16*)a.W;
+  p.in0 = (const bf16*)a.pre; p.in1 = (const bf16*)a.g;
+  p.self_gate = a.g == nullptr ? 1 : 0;
+  p.state = (bf16*)a.h; p.out0 = (bf16*)a.v; p.out1 = (bf16*)a.y;
+  return rr_launch(false, pl, p, a.sync, stream);
+}
+
+int rec_bwd_reg(const RecBwdArgs& a, cudaStream_t stream) {
+  const RecRegPlan pl = pick_rec_reg_plan(a.B, a.d);
+  if (!pl.ok) return ELMAN_ERR_UNSUPPORTED;
+  RecRegParams p{};
+  p.T = a.T; p.B = a.B; p.d = a.d;
+  p.W = (const bf16*)a.Wt;
+  p.self_gate = a.g == nullptr ? 1 : 0;
+  p.in0 = (const bf16*)(a.g != nullptr ? a.g : a.dy); p.in1 = (const bf16*)a.dy;
+  p.in2 = (const bf16*)a.h; p.in3 = (const bf16*)a.v;
+  p.state = (bf16*)a.dv; p.out0 = (bf16*)a.dg; p.db = a.db;
+  ELMAN_RETURN_IF(rr_launch(true, pl, p, a.sync, stream));
+  if (pl.groups > 1) return fold_db_rows(a.db, a.d, pl.groups, stream);
+  return ELMAN_OK;
+}
+
+}  // namespace elman

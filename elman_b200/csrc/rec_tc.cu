@@ -1145,6 +1145,13 @@ void fill_plan(const RecPlan& pl, RecTcParams& p) {
 
 }  // namespace
 
+int fold_db_rows(float* db, int d, int rows, cudaStream_t stream) {
+  fold_rows_kernel<<<(d + 255) / 256, 256, 0, stream>>>(db, d, rows);
+  count_launch(false);
+  ELMAN_CUDA_CHECK(cudaGetLastError());
+  return ELMAN_OK;
+}
+
 bool rec_tc_supported(int T, int B, int d, int bwd) { return make_plan(T, B, d, 0, bwd != 0).ok; }
 
 int rec_tc_blocks(int T, int B, int d, int compact) {
@@ -1220,11 +1227,7 @@ int rec_bwd_tc(const RecBwdArgs& a, cudaStream_t stream) {
   p.Wg = (const bf16*)a.Wt;
   p.direct_publish = options().rec_direct_publish == 1 ? 1 : 0;
   ELMAN_RETURN_IF(launch_rec_tc<true>(pl, p, a.Wt, a.dv, stream));
-  if (pl.reps > 1) {   // fold the replicas' bias-gradient rows into the first
-    fold_rows_kernel<<<(a.d + 255) / 256, 256, 0, stream>>>(a.db, a.d, pl.reps);
-    count_launch(false);
-    ELMAN_CUDA_CHECK(cudaGetLastError());
-  }
+  if (pl.reps > 1) return fold_db_rows(a.db, a.d, pl.reps, stream);
   return ELMAN_OK;
 }
 
