@@ -656,6 +656,44 @@ int elman_e0_backward(int dtype, int T, int B, int d, const void* W_x, const voi
 
 // ------------------------------- E5 ----------------------------------------
 
+// The low-rank recurrence with its factors in registers; callers that ask for the smallest
+// footprint get the single-cluster kernel where it takes the shape.
+static bool lowrank_reg_ok(int dtype, int T, int B, int d, int r, int flags) {
+  return use_tc(dtype) && lowrank_reg_supported(T, B, d, r) &&
+         !((flags & ELMAN_FLAG_COMPACT) && lowrank_tc_supported(T, B, d, r, 0) &&
+           lowrank_tc_supported(T, B, d, r, 1));
+}
+static int run_lowrank_reg_fwd(int T, int B, int d, int r, const void* U, const void* V,
+                               const void* pre, const void* gate, void* h, void* y, void* v, void* q,
+                               int rq, int* sync, cudaStream_t st) {
+  PhaseTimer timer(0, st);
+  LowRankRegArgs a{};
+  a.T = T; a.B = B; a.d = d; a.r = r; a.bwd = 0;
+  a.A1 = V; a.a1_row = d; a.a1_k = 1;
+  a.A2 = U; a.a2_row = r; a.a2_k = 1;
+  a.in0 = pre; a.in1 = gate; a.state = h; a.out0 = v; a.out1 = y;
+  a.q = q; a.rq = rq; a.sync = sync;
+  return lowrank_reg(a, st);
+}
+// dVh [T+1,B,rp]: slots 1 .. T-1 come out of the recurrence (slot T belongs to the carried-in
+// gradient), slot 0 is one more product of B rows.
+static int run_lowrank_reg_bwd(int T, int B, int d, int r, const void* U, const void* V,
+                               const void* gate, const void* dy, const void* h, const void* v,
+                               void* dv, void* dg, float* db, void* dVh, int rp, const void* Upad,
+                               int* sync, cudaStream_t st) {
+  {
+    PhaseTimer timer(1, st);
+    LowRankRegArgs a{};
+    a.T = T; a.B = B; a.d = d; a.r = r; a.bwd = 1;
+    a.A1 = U; a.a1_row = 1; a.a1_k = r;
+    a.A2 = V; a.a2_row = 1; a.a2_k = d;
+    a.in0 = gate; a.in1 = dy; a.in2 = h; a.in3 = v; a.state = dv; a.out0 = dg; a.db = db;
+    a.q = dVh; a.rq = rp; a.sync = sync;
+    ELMAN_RETURN_IF(lowrank_reg(a, st));
+  }
+  return gemm_nn(ELMAN_BF16, B, rp, d, dv, d, Upad, rp, nullptr, dVh, rp, 0, st);
+}
+
 // In the bf16 tensor-core path every factor is used zero-padded to rp = rank rounded
 // up to 64: the time-parallel GEMMs then meet the TMA alignment rules for any rank
 // (e.g. 270) and the extra columns contribute exact zeros.
@@ -702,6 +740,16 @@ int elman_e5_forward(int dtype, int training, int T, int B, int d, int r, const 
                      const void* V_x, const void* U_z, const void* V_z, const void* b, void* h,
                      void* output, void* v, void* workspace, size_t workspace_bytes,
                      void* stream) {
+  return elman_e5_forward_flags(dtype, 0, training, T, B, d, r, x, h0, U_h, V_h, U_x, V_x, U_z, V_z,
+                                b, h, output, v, workspace, workspace_bytes, stream);
+}
+
+int elman_e5_forward_flags(int dtype, int flags, int training, int T, int B, int d, int r,
+                           const void* x, const void* h0, const void* U_h, const void* V_h,
+                           const void* U_x, const void* V_x, const void* U_z, const void* V_z,
+                           const void* b, void* h, void* output, void* v, void* workspace,
+                           size_t workspace_bytes, void* stream) {
+  ELMAN_ARG_CHECK((flags & ~ELMAN_FLAG_COMPACT) == 0, "unknown flags 0x%x", flags);
   ELMAN_RETURN_IF(check_common(dtype, T, B, d));
   ELMAN_ARG_CHECK(r >= 1, "rank must be positive (got %d)", r);
   if (B == 0 || d == 0) return ELMAN_OK;
@@ -732,6 +780,11 @@ int elman_e5_forward(int dtype, int training, int T, int B, int d, int r, const 
   ELMAN_RETURN_IF(proj_nt(dtype, TB, d, rp, w.Vx, rp, Ux, rp, b, w.pre, d, 0, st));
   ELMAN_RETURN_IF(proj_nt(dtype, TB, rp, d, x, d, Vz, d, nullptr, w.Vz, rp, 0, st));
   ELMAN_RETURN_IF(proj_nt(dtype, TB, d, rp, w.Vz, rp, Uz, rp, nullptr, w.gate, d, 0, st));
+  if (lowrank_reg_ok(dtype, T, B, d, r, flags)) {   // the rank vectors go where x V_x^T was
+    const int rc = run_lowrank_reg_fwd(T, B, d, r, U_h, V_h, w.pre, w.gate, h, output,
+                                       training ? v : nullptr, w.Vx, rp, w.sync, st);
+    if (rc != ELMAN_ERR_UNSUPPORTED) return rc;
+  }
   if (use_tc(dtype) && lowrank_tc_supported(T, B, d, r, 0)) {
     LowRankTcArgs ta{};
     ta.T = T; ta.B = B; ta.d = d; ta.r = r; ta.bwd = 0;
@@ -766,7 +819,7 @@ static size_t carve_e5_bwd(int dtype, int T, int B, int d, int r, void* ws, E5Bw
   o->Vt = c.take((size_t)d * r * es);
   o->dv = c.take(TBd + (size_t)B * d * es);  // one extra time slot: the zero gradient from the future
   o->dg = c.take(TBd);
-  o->db = (float*)c.take((size_t)d * sizeof(float));
+  o->db = (float*)c.take((size_t)REC_MAX_DB_ROWS * d * sizeof(float));
   o->tmp = (float*)c.take((size_t)2 * B * r * sizeof(float));
   o->sync = (int*)c.take(rec_sync_bytes());
   o->trace = (long long*)c.take(kTraceBytes);
@@ -776,7 +829,7 @@ static size_t carve_e5_bwd(int dtype, int T, int B, int d, int r, void* ws, E5Bw
   o->Vh = c.take(TBr);
   o->dVx = c.take(TBr);
   o->dVz = c.take(TBr);
-  o->dVh = c.take(TBr);
+  o->dVh = c.take(TBr + (size_t)B * ra * es);   // one extra time slot: see run_lowrank_reg_bwd
   o->UP = o->VP = o->dUP = o->dVP = nullptr;
   for (int i = 0; i < 6; ++i) o->P[i] = nullptr;
   if (dtype == ELMAN_BF16) {
@@ -806,18 +859,31 @@ int elman_e5_backward(int dtype, int T, int B, int d, int r, const void* U_h, co
                                  workspace, workspace_bytes, stream);
 }
 
-int elman_b200_lowrank_blocks(int dtype, int T, int B, int d, int r) {
-  if (T <= 0 || B <= 0 || d <= 0 || r <= 0 || !use_tc(dtype)) return 0;
-  return lowrank_tc_supported(T, B, d, r, 0) && lowrank_tc_supported(T, B, d, r, 1)
-             ? lowrank_tc_blocks(T, B, d, r) : 0;
-}
-
 int elman_e5_backward_carry(int dtype, int T, int B, int d, int r, const void* U_h,
                             const void* V_h, const void* U_x, const void* V_x, const void* U_z,
                             const void* V_z, const void* x, const void* h, const void* v,
                             const void* d_output, const void* dv_in, void* dx, void* dU_h,
                             void* dV_h, void* dU_x, void* dV_x, void* dU_z, void* dV_z, void* db,
                             void* dv_out, void* workspace, size_t workspace_bytes, void* stream) {
+  return elman_e5_backward_carry_flags(dtype, 0, T, B, d, r, U_h, V_h, U_x, V_x, U_z, V_z, x, h, v,
+                                       d_output, dv_in, dx, dU_h, dV_h, dU_x, dV_x, dU_z, dV_z, db,
+                                       dv_out, workspace, workspace_bytes, stream);
+}
+
+int elman_b200_lowrank_blocks(int dtype, int T, int B, int d, int r) {
+  if (T <= 0 || B <= 0 || d <= 0 || r <= 0 || !use_tc(dtype)) return 0;
+  return lowrank_tc_supported(T, B, d, r, 0) && lowrank_tc_supported(T, B, d, r, 1)
+             ? lowrank_tc_blocks(T, B, d, r) : 0;
+}
+
+int elman_e5_backward_carry_flags(int dtype, int flags, int T, int B, int d, int r, const void* U_h,
+                                  const void* V_h, const void* U_x, const void* V_x,
+                                  const void* U_z, const void* V_z, const void* x, const void* h,
+                                  const void* v, const void* d_output, const void* dv_in, void* dx,
+                                  void* dU_h, void* dV_h, void* dU_x, void* dV_x, void* dU_z,
+                                  void* dV_z, void* db, void* dv_out, void* workspace,
+                                  size_t workspace_bytes, void* stream) {
+  ELMAN_ARG_CHECK((flags & ~ELMAN_FLAG_COMPACT) == 0, "unknown flags 0x%x", flags);
   ELMAN_RETURN_IF(check_common(dtype, T, B, d));
   ELMAN_ARG_CHECK(r >= 1, "rank must be positive (got %d)", r);
   if (d == 0) return ELMAN_OK;
@@ -862,8 +928,6 @@ int elman_e5_backward_carry(int dtype, int T, int B, int d, int r, const void* U
   // recompute the gate pre-activation (the reference does the same per step)
   ELMAN_RETURN_IF(proj_nt(dtype, TB, rp, d, x, d, Vz, d, nullptr, w.Vz, rp, 0, st));
   ELMAN_RETURN_IF(proj_nt(dtype, TB, d, rp, w.Vz, rp, Uz, rp, nullptr, w.gate, d, 0, st));
-  ELMAN_RETURN_IF(transpose2d(dtype, d, r, U_h, w.Ut, st));  // [r,d]
-  ELMAN_RETURN_IF(transpose2d(dtype, r, d, V_h, w.Vt, st));  // [d,r]
   {  // slot T of dv: the pre-activation gradient of the step after this call's last one
     const size_t slot = (size_t)B * d * es;
     char* last = (char*)w.dv + (size_t)T * slot;
@@ -872,19 +936,29 @@ int elman_e5_backward_carry(int dtype, int T, int B, int d, int r, const void* U
     else
       ELMAN_CUDA_CHECK(cudaMemsetAsync(last, 0, slot, st));
   }
-  if (use_tc(dtype) && lowrank_tc_supported(T, B, d, r, 1)) {
-    // dh_rec = (dv U) V: first product with U^T [r,d], second with V^T [d,r]
-    LowRankTcArgs ta{};
-    ta.T = T; ta.B = B; ta.d = d; ta.r = r; ta.bwd = 1;
-    ta.Urole = w.Vt; ta.Vrole = w.Ut;
-    ta.in0 = w.gate; ta.in1 = d_output; ta.in2 = h; ta.in3 = v;
-    ta.state = w.dv; ta.out0 = w.dg; ta.out1 = nullptr; ta.db = w.db;
-    ta.UP = w.UP; ta.VP = w.VP; ta.sync = w.sync; ta.trace = w.trace;
-    ELMAN_RETURN_IF(lowrank_tc(ta, st));
-  } else {
-    LowRankBwdArgs a{T, B, d, r, w.Ut, w.Vt, h, v, w.gate, d_output, w.dv, w.dg, w.db, w.tmp,
-                     w.sync};
-    ELMAN_RETURN_IF(lowrank_bwd_generic(dtype, a, st));
+  int rec = ELMAN_ERR_UNSUPPORTED;
+  if (lowrank_reg_ok(dtype, T, B, d, r, flags))
+    rec = run_lowrank_reg_bwd(T, B, d, r, U_h, V_h, w.gate, d_output, h, v, w.dv, w.dg, w.db, w.dVh,
+                              rp, Uh, w.sync, st);
+  const bool have_dVh = rec == ELMAN_OK;
+  if (rec != ELMAN_OK && rec != ELMAN_ERR_UNSUPPORTED) return rec;
+  if (!have_dVh) {
+    ELMAN_RETURN_IF(transpose2d(dtype, d, r, U_h, w.Ut, st));  // [r,d]
+    ELMAN_RETURN_IF(transpose2d(dtype, r, d, V_h, w.Vt, st));  // [d,r]
+    if (use_tc(dtype) && lowrank_tc_supported(T, B, d, r, 1)) {
+      // dh_rec = (dv U) V: first product with U^T [r,d], second with V^T [d,r]
+      LowRankTcArgs ta{};
+      ta.T = T; ta.B = B; ta.d = d; ta.r = r; ta.bwd = 1;
+      ta.Urole = w.Vt; ta.Vrole = w.Ut;
+      ta.in0 = w.gate; ta.in1 = d_output; ta.in2 = h; ta.in3 = v;
+      ta.state = w.dv; ta.out0 = w.dg; ta.out1 = nullptr; ta.db = w.db;
+      ta.UP = w.UP; ta.VP = w.VP; ta.sync = w.sync; ta.trace = w.trace;
+      ELMAN_RETURN_IF(lowrank_tc(ta, st));
+    } else {
+      LowRankBwdArgs a{T, B, d, r, w.Ut, w.Vt, h, v, w.gate, d_output, w.dv, w.dg, w.db, w.tmp,
+                       w.sync};
+      ELMAN_RETURN_IF(lowrank_bwd_generic(dtype, a, st));
+    }
   }
   if (dv_out != nullptr)
     ELMAN_CUDA_CHECK(cudaMemcpyAsync(dv_out, w.dv, (size_t)B * d * es, cudaMemcpyDeviceToDevice, st));
@@ -894,7 +968,8 @@ int elman_e5_backward_carry(int dtype, int T, int B, int d, int r, const void* U
   ELMAN_RETURN_IF(proj_nt(dtype, TB, rp, d, h, d, Vh, d, nullptr, w.Vh, rp, 0, st));
   ELMAN_RETURN_IF(gemm_nn(dtype, TB, rp, d, w.dv, d, Ux, rp, nullptr, w.dVx, rp, 0, st));
   ELMAN_RETURN_IF(gemm_nn(dtype, TB, rp, d, w.dg, d, Uz, rp, nullptr, w.dVz, rp, 0, st));
-  ELMAN_RETURN_IF(gemm_nn(dtype, TB, rp, d, w.dv, d, Uh, rp, nullptr, w.dVh, rp, 0, st));
+  if (!have_dVh)
+    ELMAN_RETURN_IF(gemm_nn(dtype, TB, rp, d, w.dv, d, Uh, rp, nullptr, w.dVh, rp, 0, st));
   // dx = dVx V_x + dVz V_z
   ELMAN_RETURN_IF(gemm_nn(dtype, TB, d, rp, w.dVx, rp, Vx, d, nullptr, dx, d, 0, st));
   ELMAN_RETURN_IF(gemm_nn(dtype, TB, d, rp, w.dVz, rp, Vz, d, nullptr, dx, d, 1, st));
@@ -924,12 +999,13 @@ int elman_e5_backward_carry(int dtype, int T, int B, int d, int r, const void* U
 // projection of x and with z as the gate input; the time-parallel part is E1's.
 
 struct E4FwdWs {
-  void* pre; float* tmp; int* sync; long long* trace; void* UP; void* VP;
+  void* q; void* pre; float* tmp; int* sync; long long* trace; void* UP; void* VP;
 };
 static size_t carve_e4_fwd(int dtype, int T, int B, int d, int r, void* ws, E4FwdWs* o) {
   Carver c(ws);
   size_t es = esize(dtype);
   o->pre = c.take((size_t)T * B * d * es);
+  o->q = c.take((size_t)T * B * e5_rank_alloc(dtype, r) * es);   // rank vectors
   o->tmp = (float*)c.take((size_t)2 * B * r * sizeof(float));
   o->sync = (int*)c.take(rec_sync_bytes());
   o->trace = (long long*)c.take(kTraceBytes);
@@ -968,6 +1044,11 @@ int elman_e4_forward(int dtype, int training, int T, int B, int d, int r, const 
   if (workspace_bytes < need)
     return set_error(ELMAN_ERR_WORKSPACE, "workspace %zu < required %zu", workspace_bytes, need);
   ELMAN_RETURN_IF(proj_nt(dtype, T * B, d, d, x, d, W_x, d, b, w.pre, d, 0, st));
+  if (lowrank_reg_ok(dtype, T, B, d, r, 0)) {
+    const int rc = run_lowrank_reg_fwd(T, B, d, r, U, V, w.pre, z, h, output, training ? v : nullptr,
+                                       w.q, e5_rank_run(dtype, r), w.sync, st);
+    if (rc != ELMAN_ERR_UNSUPPORTED) return rc;
+  }
   if (use_tc(dtype) && lowrank_tc_supported(T, B, d, r, 0)) {
     LowRankTcArgs ta{};
     ta.T = T; ta.B = B; ta.d = d; ta.r = r; ta.bwd = 0;
@@ -994,14 +1075,14 @@ static size_t carve_e4_bwd(int dtype, int T, int B, int d, int r, void* ws, E4Bw
   o->Ut = c.take((size_t)d * r * es);
   o->Vt = c.take((size_t)d * r * es);
   o->dv = c.take(TBd + (size_t)B * d * es);  // one extra time slot: the zero gradient from the future
-  o->db = (float*)c.take((size_t)d * sizeof(float));
+  o->db = (float*)c.take((size_t)REC_MAX_DB_ROWS * d * sizeof(float));
   o->tmp = (float*)c.take((size_t)2 * B * r * sizeof(float));
   o->sync = (int*)c.take(rec_sync_bytes());
   o->trace = (long long*)c.take(kTraceBytes);
   o->splitk_bytes = splitk_scratch_bytes(dtype, d, d);
   o->splitk = o->splitk_bytes ? (float*)c.take(o->splitk_bytes) : nullptr;
   o->Vh = c.take(TBr);
-  o->dVh = c.take(TBr);
+  o->dVh = c.take(TBr + (size_t)B * ra * es);   // one extra time slot: see run_lowrank_reg_bwd
   o->UP = o->VP = o->UhP = o->VhP = o->dUP = o->dVP = nullptr;
   if (dtype == ELMAN_BF16) {
     size_t up = 0, vp = 0;
@@ -1054,27 +1135,36 @@ int elman_e4_backward(int dtype, int T, int B, int d, int r, const void* W_x, co
     ELMAN_RETURN_IF(resize2d(dtype, V, r, d, w.VhP, rp, d, st));
     Uh = w.UhP; Vh = w.VhP;
   }
-  ELMAN_RETURN_IF(transpose2d(dtype, d, r, U, w.Ut, st));  // [r,d]
-  ELMAN_RETURN_IF(transpose2d(dtype, r, d, V, w.Vt, st));  // [d,r]
   ELMAN_CUDA_CHECK(cudaMemsetAsync((char*)w.dv + (size_t)T * B * d * es, 0, (size_t)B * d * es, st));
-  if (use_tc(dtype) && lowrank_tc_supported(T, B, d, r, 1)) {
-    LowRankTcArgs ta{};
-    ta.T = T; ta.B = B; ta.d = d; ta.r = r; ta.bwd = 1;
-    ta.Urole = w.Vt; ta.Vrole = w.Ut;
-    ta.in0 = z; ta.in1 = d_output; ta.in2 = h; ta.in3 = v;
-    ta.state = w.dv; ta.out0 = dz; ta.out1 = nullptr; ta.db = w.db;
-    ta.UP = w.UP; ta.VP = w.VP; ta.sync = w.sync; ta.trace = w.trace;
-    ELMAN_RETURN_IF(lowrank_tc(ta, st));
-  } else {
-    LowRankBwdArgs a{T, B, d, r, w.Ut, w.Vt, h, v, z, d_output, w.dv, dz, w.db, w.tmp, w.sync};
-    ELMAN_RETURN_IF(lowrank_bwd_generic(dtype, a, st));
+  int rec = ELMAN_ERR_UNSUPPORTED;
+  if (lowrank_reg_ok(dtype, T, B, d, r, 0))
+    rec = run_lowrank_reg_bwd(T, B, d, r, U, V, z, d_output, h, v, w.dv, dz, w.db, w.dVh, rp, Uh, w.sync,
+                              st);
+  const bool have_dVh = rec == ELMAN_OK;
+  if (rec != ELMAN_OK && rec != ELMAN_ERR_UNSUPPORTED) return rec;
+  if (!have_dVh) {
+    ELMAN_RETURN_IF(transpose2d(dtype, d, r, U, w.Ut, st));  // [r,d]
+    ELMAN_RETURN_IF(transpose2d(dtype, r, d, V, w.Vt, st));  // [d,r]
+    if (use_tc(dtype) && lowrank_tc_supported(T, B, d, r, 1)) {
+      LowRankTcArgs ta{};
+      ta.T = T; ta.B = B; ta.d = d; ta.r = r; ta.bwd = 1;
+      ta.Urole = w.Vt; ta.Vrole = w.Ut;
+      ta.in0 = z; ta.in1 = d_output; ta.in2 = h; ta.in3 = v;
+      ta.state = w.dv; ta.out0 = dz; ta.out1 = nullptr; ta.db = w.db;
+      ta.UP = w.UP; ta.VP = w.VP; ta.sync = w.sync; ta.trace = w.trace;
+      ELMAN_RETURN_IF(lowrank_tc(ta, st));
+    } else {
+      LowRankBwdArgs a{T, B, d, r, w.Ut, w.Vt, h, v, z, d_output, w.dv, dz, w.db, w.tmp, w.sync};
+      ELMAN_RETURN_IF(lowrank_bwd_generic(dtype, a, st));
+    }
   }
   ELMAN_RETURN_IF(float_to_dtype(dtype, w.db, db, d, st));
   // time-parallel part: dx = dv W_x, dW_x = dv^T x; rank activations Vh = h V^T, dVh = dv U
   ELMAN_RETURN_IF(gemm_nn(dtype, TB, d, d, w.dv, d, W_x, d, nullptr, dx, d, 0, st));
   ELMAN_RETURN_IF(gemm_tn(dtype, d, d, TB, w.dv, x, dW_x, st, w.splitk, w.splitk_bytes));
   ELMAN_RETURN_IF(proj_nt(dtype, TB, rp, d, h, d, Vh, d, nullptr, w.Vh, rp, 0, st));
-  ELMAN_RETURN_IF(gemm_nn(dtype, TB, rp, d, w.dv, d, Uh, rp, nullptr, w.dVh, rp, 0, st));
+  if (!have_dVh)
+    ELMAN_RETURN_IF(gemm_nn(dtype, TB, rp, d, w.dv, d, Uh, rp, nullptr, w.dVh, rp, 0, st));
   {  // dU [d, r] = dv^T [d, TB] * Vh [TB, rp]
     void* out = padded ? w.dUP : dU;
     ELMAN_RETURN_IF(gemm_tn(dtype, d, rp, TB, w.dv, w.Vh, out, st, w.splitk, w.splitk_bytes));

@@ -246,7 +246,7 @@ int lowrank_bwd_generic(int dtype, const LowRankBwdArgs& a, cudaStream_t stream)
 constexpr int REC_MAX_REPLICAS = 4;
 // Rows of bias-gradient sums (one per replica or batch group) a recurrence may write before they
 // are folded into the first.
-constexpr int REC_MAX_DB_ROWS = 16;
+constexpr int REC_MAX_DB_ROWS = 32;
 int fold_db_rows(float* db, int d, int rows, cudaStream_t stream);
 bool rec_tc_supported(int T, int B, int d, int bwd);   // per direction: the plans differ
 // resident thread blocks of one launch (compact: smallest-footprint plan), 0 if unsupported
@@ -263,6 +263,27 @@ bool rec_reg_supported(int T, int B, int d);
 int rec_reg_blocks(int B, int d);
 int rec_fwd_reg(const RecFwdArgs& a, cudaStream_t stream);
 int rec_bwd_reg(const RecBwdArgs& a, cudaStream_t stream);
+int rec_reg_sms();   // multiprocessors of the current device
+
+// Low-rank recurrence, bf16, both factors in registers (lowrank_reg.cuh): d % 8 == 0, d from 64 to
+// 2048, rank up to 512.
+//   forward : in0 = pre, in1 = gate, state = h [T+1,B,d] (h[0] filled), out0 = v (or null), out1 = y,
+//             A1 = V [r,d], A2 = U [d,r];  q [T,B,rq] receives V h_{t-1} of every step t
+//   backward: in0 = gate, in1 = dy, in2 = h, in3 = v, state = dv [T+1,B,d] (slot T filled), out0 = dg,
+//             db fp32 [REC_MAX_DB_ROWS, d], A1 = U^T, A2 = V^T;  q [T+1,B,rq]: slot t receives U^T dv_t
+//             for t = T .. 1
+// Factors are read through strides: element (row, k) of A at row * a_row + k * a_k.
+struct LowRankRegArgs {
+  int T, B, d, r, bwd;
+  const void* A1; long a1_row, a1_k;
+  const void* A2; long a2_row, a2_k;
+  const void* in0; const void* in1; const void* in2; const void* in3;
+  void* state; void* out0; void* out1; float* db;
+  void* q; int rq;
+  int* sync;
+};
+bool lowrank_reg_supported(int T, int B, int d, int r);
+int lowrank_reg(const LowRankRegArgs& a, cudaStream_t stream);
 
 // Copies the cycle stamps of the last traced launch (option rec_trace) to the host.
 int rec_tc_copy_trace(long long* dst, int max_entries);

@@ -15,16 +15,6 @@ struct RecRegPlan {
   bool ok;
 };
 
-int device_sms() {
-  static int sms[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return 0; }
-  if (sms[dev] == 0 &&
-      cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    cudaGetLastError();
-  return sms[dev];
-}
-
 // MB of state that one look of all CTAs together reads.
 double rr_look_mb(int B, int d, int cpg) { return (double)B * d * 2 * cpg / 1e6; }
 
@@ -59,7 +49,7 @@ RecRegPlan pick_rec_reg_plan(int B, int d) {
   best.ok = false;
   const int kb = ((d + 31) / 32 + RR_WARPS - 1) / RR_WARPS;
   if (B < 1 || B > RR_MAX_BATCH || d < 8 || (d & 7) != 0 || kb > RR_MAX_KB) return best;
-  const int sms = device_sms();
+  const int sms = rec_reg_sms();
   double best_cost = 0;
   for (int pass = 0; pass < 2; ++pass) {
     int best_ctas = 0;
@@ -102,6 +92,7 @@ int rr_launch(bool bwd, const RecRegPlan& pl, RecRegParams& p, int* sync, cudaSt
   const size_t smem = rec_reg_smem(bwd, pl.mt, pl.nt);
   if (smem > 48 * 1024)
     ELMAN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  p.b_lo = 0; p.b_hi = p.B;
   p.cpg = pl.cpg;
   p.hold = rr_hold(p.B, p.d, pl.cpg);
   p.abort_word = sync;
@@ -131,6 +122,16 @@ int rr_launch(bool bwd, const RecRegPlan& pl, RecRegParams& p, int* sync, cudaSt
 }
 
 }  // namespace
+
+int rec_reg_sms() {
+  static int sms[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return 0; }
+  if (sms[dev] == 0 &&
+      cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    cudaGetLastError();
+  return sms[dev];
+}
 
 bool rec_reg_supported(int T, int B, int d) {
   return T >= 1 && rr_enabled() && pick_rec_reg_plan(B, d).ok;

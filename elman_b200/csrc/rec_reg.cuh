@@ -56,6 +56,7 @@ inline size_t rec_reg_smem(bool bwd, int mt, int nt) {
 
 struct RecRegParams {
   int T, B, d;
+  int b_lo, b_hi;         // batch rows of this launch
   int cpg;                // CTAs per batch group
   const bf16* W;          // [d, d], row = output feature (backward: the transposed matrix)
   const bf16* in0;        // forward pre            backward g
@@ -123,37 +124,282 @@ __device__ __forceinline__ uint32_t pack(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
+// One look at a lane's fragments of the state: KB blocks of 32 columns for each of NT row tiles.
+template <int NT, int KB>
+__device__ __forceinline__ void look(uint4 (&x)[NT][KB], const char* src, const uint32_t (&x_off)[NT]) {
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int kb = 0; kb < KB; ++kb) x[nt][kb] = ld_relaxed_v4(src + x_off[nt] + kb * 64);
+}
+
+// Looks again at what was not there yet until all of it is; false when the wait gave up.
+// `stalled` (test hook): never satisfied.
+template <int NT, int KB>
+__device__ __forceinline__ bool await(uint4 (&x)[NT][KB], const char* src, const uint32_t (&x_off)[NT],
+                                      bool stalled, long spin_limit, const int* abort_word) {
+  long spins = 0;
+  unsigned long long t_begin = 0;
+  while (true) {
+    // one comparison for everything: the pattern is the largest unsigned value
+    uint32_t top = stalled ? 0xFFFFFFFFu : 0u;
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int kb = 0; kb < KB; ++kb) top = max(top, largest(x[nt][kb]));
+    if (top != 0xFFFFFFFFu) return true;
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int kb = 0; kb < KB; ++kb)
+        if (largest(x[nt][kb]) == 0xFFFFFFFFu) x[nt][kb] = ld_relaxed_v4(src + x_off[nt] + kb * 64);
+    if (++spins > spin_limit) return false;
+    if ((spins & 63) == 0) {
+      const unsigned long long now = ptx::globaltimer_ns();
+      if (t_begin == 0) t_begin = now;
+      if (ld_relaxed_gpu(abort_word) != 0 || now - t_begin > ptx::kWaitDeadlineNs) return false;
+    }
+  }
+}
+
+// The products of one warp: acc[mt][nt] += W tile mt (A fragments) times the state's row tile nt
+// over KB blocks of two k-steps.
+template <int CH, int MT, int NT, int KB>
+__device__ __forceinline__ void products(float (&acc)[CH][MT][NT][4], const uint32_t (&w)[MT][KB][8],
+                                         const uint4 (&x)[NT][KB]) {
+#pragma unroll
+  for (int ch = 0; ch < CH; ++ch)
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[ch][mt][nt][u] = 0.f;
+#pragma unroll
+  for (int kb = 0; kb < KB; ++kb) {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+        mma_bf16(acc[0][mt][nt], w[mt][kb][0], w[mt][kb][1], w[mt][kb][2], w[mt][kb][3], x[nt][kb].x,
+                 x[nt][kb].y);
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+        mma_bf16(acc[CH - 1][mt][nt], w[mt][kb][4], w[mt][kb][5], w[mt][kb][6], w[mt][kb][7],
+                 x[nt][kb].z, x[nt][kb].w);
+  }
+}
+
+// A warp's accumulators to its part of the partial-sum buffer [NT * 8 rows][stride].
+template <int CH, int MT, int NT>
+__device__ __forceinline__ void put_partials(float* dst, int stride, int gq, int tq,
+                                             const float (&acc)[CH][MT][NT][4]) {
+  float* mine = dst + 2 * tq * stride + gq;
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float v = acc[0][mt][nt][u];
+        if (CH == 2) v += acc[1][mt][nt][u];
+        mine[(nt * 8 + (u & 1)) * stride + mt * 16 + 8 * (u >> 1)] = v;
+      }
+}
+
+// Sum over the warps' partial sums of a feature pair.
+__device__ __forceinline__ float2 gather_pair(const float* at, int warp_stride) {
+  float2 q[RR_WARPS];
+#pragma unroll
+  for (int wv = 0; wv < RR_WARPS; ++wv) q[wv] = *reinterpret_cast<const float2*>(at + wv * warp_stride);
+#pragma unroll
+  for (int st = 1; st < RR_WARPS; st *= 2)
+#pragma unroll
+    for (int wv = 0; wv < RR_WARPS; wv += 2 * st) { q[wv].x += q[wv + st].x; q[wv].y += q[wv + st].y; }
+  return q[0];
+}
+
+// The part of a step behind the products, for one thread: the feature pairs it finishes, their
+// inputs (a ring of asynchronous copies) and their outputs.
+template <bool BWD, int R, int NG>
+struct Tail {
+  static constexpr int PS = R + 4;       // row stride of the partial sums: conflict-free stores
+  static constexpr int PAIRS = R / 2;
+  static constexpr int ITEMS = (PAIRS * NG + RR_THREADS - 1) / RR_THREADS;   // pairs per thread
+  static constexpr int NIN = BWD ? 4 : 2;
+  const RecRegParams& p;
+  const int slot;         // bytes of one time slot
+  uint32_t* const ring;
+  uint32_t off[ITEMS];    // byte offset inside one [B, d] slot
+  int spart[ITEMS];       // offset of the pair's partial sums
+  bool mine[ITEMS];
+  // what does not depend on the recurrent term: forward e0 = pre, e1 = silu(g);
+  // backward e0 = dy silu(g), e1 = 1 - tanh(v)^2, late = dg
+  float2 e0[ITEMS], e1[ITEMS], dbs[ITEMS];
+  uint32_t late[ITEMS], o0[ITEMS], o1[ITEMS];
+
+  __device__ __forceinline__ Tail(const RecRegParams& p_, float* ring_area, int f0, int b0)
+      : p(p_), slot(p_.B * p_.d * 2), ring(reinterpret_cast<uint32_t*>(ring_area) + threadIdx.x) {
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const int e = threadIdx.x + i * RR_THREADS;
+      const int n = e / PAIRS, f = 2 * (e - n * PAIRS);
+      mine[i] = e < PAIRS * NG && f0 + f < p.d && b0 + n < p.b_hi;
+      spart[i] = mine[i] ? n * PS + f : 0;
+      off[i] = mine[i] ? (uint32_t)((b0 + n) * p.d + f0 + f) * 2u : 0u;
+      dbs[i] = make_float2(0.f, 0.f);
+    }
+  }
+  static __device__ __forceinline__ const unsigned int* word(const bf16* base, long at, uint32_t off) {
+    return reinterpret_cast<const unsigned int*>(reinterpret_cast<const char*>(base) + at + off);
+  }
+  __device__ __forceinline__ uint32_t* slot_of(int s, int i, int k) const {
+    return ring + (((s & (RR_AHEAD - 1)) * ITEMS + i) * NIN + k) * RR_THREADS;
+  }
+  // Inputs of step s (time slot at byte `at`).  Each thread copies its own words, RR_AHEAD - 1
+  // steps ahead: loads into registers would share the scoreboards that the looks at the state
+  // wait on, and tie the chain to DRAM.
+  __device__ __forceinline__ void fetch(int s, long at) {
+    if (s < p.T) {
+#pragma unroll
+      for (int i = 0; i < ITEMS; ++i)
+        if (mine[i]) {
+          copy_word(slot_of(s, i, 0), word(p.in0, at, off[i]));
+          if (BWD || !p.self_gate) copy_word(slot_of(s, i, 1), word(p.in1, at, off[i]));
+          if (BWD) {
+            copy_word(slot_of(s, i, 2), word(p.in2, at + slot, off[i]));
+            copy_word(slot_of(s, i, 3), word(p.in3, at, off[i]));
+          }
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  __device__ __forceinline__ void premath(int s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(RR_AHEAD - 1) : "memory");
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      if (!mine[i]) continue;
+      uint32_t raw[NIN];
+#pragma unroll
+      for (int k = 0; k < NIN; ++k) raw[k] = *slot_of(s, i, k);
+      if (!BWD) {
+        e0[i] = unpack(raw[0]);
+        if (!p.self_gate) {
+          const float2 g = unpack(raw[1]);
+          e1[i] = make_float2(g.x * sigmoid_fast(g.x), g.y * sigmoid_fast(g.y));
+        }
+      } else {
+        float2 g = unpack(raw[0]);
+        const float2 dy = unpack(raw[1]), h = unpack(raw[NIN - 2]), v = unpack(raw[NIN - 1]);
+        if (p.self_gate) g = h;
+        const float sx = sigmoid_fast(g.x), sy = sigmoid_fast(g.y);
+        const float gx = dy.x * h.x * sx * (1.f + g.x * (1.f - sx));
+        const float gy = dy.y * h.y * sy * (1.f + g.y * (1.f - sy));
+        late[i] = pack(gx, gy);
+        e0[i] = make_float2(dy.x * g.x * sx, dy.y * g.y * sy);
+        if (p.self_gate) { e0[i].x += gx; e0[i].y += gy; }   // d(h silu(h))/dh = silu(h) + h silu'(h)
+        e1[i] = make_float2(dtanh_from_v(v.x), dtanh_from_v(v.y));
+      }
+      // computed now, not sunk to their use behind the wait
+      asm volatile("" : "+f"(e0[i].x), "+f"(e0[i].y), "+f"(e1[i].x), "+f"(e1[i].y));
+      if (BWD) asm volatile("" : "+r"(late[i]));
+    }
+  }
+  // The new state of the step whose time slot is at byte `at`, from the partial sums in `buf`.
+  __device__ __forceinline__ void publish(const float* buf, long at) {
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      if (!mine[i]) continue;
+      float2 a = gather_pair(buf + spart[i], NG * PS);
+      char* dst = reinterpret_cast<char*>(p.state) + (BWD ? at : at + slot) + off[i];
+      if (!BWD) {
+        a.x += e0[i].x; a.y += e0[i].y;
+        const float h0 = tanh_fast(a.x), h1 = tanh_fast(a.y);
+        const uint32_t hp = pack(h0, h1);
+        st_relaxed_u32(dst, hp);
+        o0[i] = pack(a.x, a.y);
+        if (p.self_gate) {     // the gate is the state as stored
+          const float2 hs = unpack(hp);
+          o1[i] = pack(h0 * hs.x * sigmoid_fast(hs.x), h1 * hs.y * sigmoid_fast(hs.y));
+        } else {
+          o1[i] = pack(h0 * e1[i].x, h1 * e1[i].y);
+        }
+      } else {
+        const float d0 = (e0[i].x + a.x) * e1[i].x, d1 = (e0[i].y + a.y) * e1[i].y;
+        st_relaxed_u32(dst, pack(d0, d1));
+        dbs[i].x += d0; dbs[i].y += d1;
+        o0[i] = late[i];
+      }
+    }
+  }
+  // Outputs that no other CTA waits for.
+  __device__ __forceinline__ void store_rest(long at) {
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      if (!mine[i]) continue;
+      if (p.out0 != nullptr) *const_cast<unsigned int*>(word(p.out0, at, off[i])) = o0[i];
+      if (!BWD) *const_cast<unsigned int*>(word(p.out1, at, off[i])) = o1[i];
+    }
+  }
+  // Bias gradient of the group's rows, in a fixed order (all threads; reuses the partial sums).
+  __device__ __forceinline__ void fold_bias(float* part, int f0, int grp) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const int e = threadIdx.x + i * RR_THREADS, n = e / PAIRS;
+      if (e < PAIRS * NG) *reinterpret_cast<float2*>(part + n * PS + 2 * (e - n * PAIRS)) = dbs[i];
+    }
+    __syncthreads();
+    if (threadIdx.x < R && f0 + (int)threadIdx.x < p.d) {
+      float sum = 0.f;
+#pragma unroll
+      for (int n = 0; n < NG; ++n) sum += part[n * PS + threadIdx.x];
+      p.db[(long)grp * p.d + f0 + threadIdx.x] = sum;
+    }
+  }
+};
+
+// The columns a lane reads: the warps' ranges of KB blocks cover [0, K) from the left; one that
+// would reach past K is moved back and its columns that another warp owns get zero weights, so
+// every look is in range without a predicate (K >= 32 KB, or KB = 1).  Lane tq takes columns 8 tq .. 8 tq + 7 of a block
+// as fragment elements (k-step 0: b0, b1; k-step 1: b0, b1), two columns each.
+template <int KB>
+struct KRange {
+  int own;      // first column that is this warp's
+  int col;      // this lane's column in the first block
+  bool any;     // false only when K < 32 leaves this lane nothing
+  __device__ __forceinline__ KRange(int K, int warp, int tq) {
+    own = warp * (KB * 32);
+    col = min(own, max(0, K - KB * 32)) + tq * 8;
+    any = col < K;
+    if (!any) col = 0;
+  }
+  __device__ __forceinline__ bool owns(int kb) const { return any && col + kb * 32 >= own; }
+};
+
 }  // namespace rr
 
 template <bool BWD, int MT, int KB, int NT>
 __global__ void __launch_bounds__(RR_THREADS, 1) rec_reg_kernel(const RecRegParams p) {
   constexpr int R = 16 * MT;             // rows of W (features) of this CTA
   constexpr int NG = 8 * NT;             // batch rows of the group
-  constexpr int PS = R + 4;              // row stride of the partial sums: conflict-free stores
-  constexpr int PAIRS = R / 2;
-  constexpr int ITEMS = (PAIRS * NG + RR_THREADS - 1) / RR_THREADS;   // feature pairs per thread
   constexpr int CH = MT * NT == 1 ? 2 : 1;   // accumulator chains when one tile alone would serialise
-  constexpr int NIN = BWD ? 4 : 2;
-  extern __shared__ __align__(16) float part[];   // [2][warps][NG][PS]
+  typedef rr::Tail<BWD, R, NG> Tail;
+  constexpr int PS = Tail::PS;
+  extern __shared__ __align__(16) float part[];   // [2][warps][NG][PS], then the ring of inputs
   __shared__ int s_bad[2];                        // a wait of an even / odd step gave up
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int gq = lane >> 2, tq = lane & 3;
-  const int T = p.T, B = p.B, d = p.d;
+  const int T = p.T, d = p.d;
   const int grp = blockIdx.x / p.cpg, c = blockIdx.x - grp * p.cpg;
-  const int f0 = c * R, b0 = grp * NG;
-  const int slot = B * d * 2;                     // bytes of one time slot
+  const int f0 = c * R, b0 = p.b_lo + grp * NG;
   if (tid < 2) s_bad[tid] = 0;
 
   // ---- my part of W, once: rows f0 .. f0+R, this warp's KB blocks of 32 columns ----
-  // Lane (gq, tq) takes columns 8 tq .. 8 tq + 7 of a block as fragment elements (k-step 0: b0, b1;
-  // k-step 1: b0, b1), two columns each.  The warps' ranges cover [0, d) from the left; one that
-  // would reach past d is moved back and its columns that another warp owns get zero weights, so
-  // every load of the step loop is in range without a predicate.
-  const int k_own = warp * (KB * 32);             // first column that is this warp's
-  int kc = min(k_own, max(0, d - KB * 32)) + tq * 8;
-  const bool k_any = kc < d;                      // false only below 32 features
-  if (!k_any) kc = 0;
+  const rr::KRange<KB> k(d, warp, tq);
   uint32_t w[MT][KB][8];
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt)
@@ -163,8 +409,8 @@ __global__ void __launch_bounds__(RR_THREADS, 1) rec_reg_kernel(const RecRegPara
       for (int u = 0; u < 2; ++u) {
         const int row = f0 + mt * 16 + gq + 8 * u;
         uint4 x = make_uint4(0, 0, 0, 0);
-        if (row < d && k_any && kc + kb * 32 >= k_own)
-          x = __ldg(reinterpret_cast<const uint4*>(p.W + (long)row * d + kc + kb * 32));
+        if (row < d && k.owns(kb))
+          x = __ldg(reinterpret_cast<const uint4*>(p.W + (long)row * d + k.col + kb * 32));
         w[mt][kb][0 + u] = x.x; w[mt][kb][2 + u] = x.y;
         w[mt][kb][4 + u] = x.z; w[mt][kb][6 + u] = x.w;
       }
@@ -172,241 +418,49 @@ __global__ void __launch_bounds__(RR_THREADS, 1) rec_reg_kernel(const RecRegPara
   uint32_t x_off[NT];
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt)
-    x_off[nt] = (uint32_t)(min(b0 + nt * 8 + gq, B - 1) * d + kc) * 2u;
+    x_off[nt] = (uint32_t)(min(b0 + nt * 8 + gq, p.b_hi - 1) * d + k.col) * 2u;
 
-  // ---- the feature pairs this thread finishes ----
-  uint32_t off[ITEMS];  // byte offset inside one [B, d] slot
-  int spart[ITEMS];     // offset of the pair's partial sums
-  bool mine[ITEMS];
-#pragma unroll
-  for (int i = 0; i < ITEMS; ++i) {
-    const int e = tid + i * RR_THREADS;
-    const int n = e / PAIRS, f = 2 * (e - n * PAIRS);
-    mine[i] = e < PAIRS * NG && f0 + f < d && b0 + n < B;
-    spart[i] = mine[i] ? n * PS + f : 0;
-    off[i] = mine[i] ? (uint32_t)((b0 + n) * d + f0 + f) * 2u : 0u;
-  }
-  // running byte positions of the step's slot in [T]-shaped tensors
+  Tail tail(p, part + 2 * RR_WARPS * NG * PS, f0, b0);
+  // running byte position of the step's slot in [T]-shaped tensors
+  const int slot = tail.slot;
   const long step_bytes = BWD ? -(long)slot : (long)slot;
   long at = BWD ? (long)(T - 1) * slot : 0;
-  auto word = [](const bf16* base, long at, uint32_t off) {
-    return reinterpret_cast<const unsigned int*>(reinterpret_cast<const char*>(base) + at + off);
-  };
-  // Inputs of later steps come in by asynchronous copies, each thread its own words, into a ring
-  // of RR_AHEAD steps: loads into registers would share the scoreboards that the looks at the
-  // state wait on, and tie the chain to DRAM.
-  uint32_t* const ring = reinterpret_cast<uint32_t*>(part + 2 * RR_WARPS * NG * PS) + tid;
-  auto slot_of = [&](int s, int i, int k) {
-    return ring + (((s & (RR_AHEAD - 1)) * ITEMS + i) * NIN + k) * RR_THREADS;
-  };
-  auto fetch = [&](int s, long at) {
-    if (s < T) {
 #pragma unroll
-      for (int i = 0; i < ITEMS; ++i)
-        if (mine[i]) {
-          rr::copy_word(slot_of(s, i, 0), word(p.in0, at, off[i]));
-          if (BWD || !p.self_gate) rr::copy_word(slot_of(s, i, 1), word(p.in1, at, off[i]));
-          if (BWD) {
-            rr::copy_word(slot_of(s, i, 2), word(p.in2, at + slot, off[i]));
-            rr::copy_word(slot_of(s, i, 3), word(p.in3, at, off[i]));
-          }
-        }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  // what does not depend on the recurrent term: forward e0 = pre, e1 = silu(g);
-  // backward e0 = dy silu(g), e1 = 1 - tanh(v)^2, late = dg
-  float2 e0[ITEMS], e1[ITEMS];
-  uint32_t late[ITEMS];
-  auto premath = [&](int s) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(RR_AHEAD - 1) : "memory");
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-      if (!mine[i]) continue;
-      uint32_t raw[NIN];
-#pragma unroll
-      for (int k = 0; k < NIN; ++k) raw[k] = *slot_of(s, i, k);
-      if (!BWD) {
-        e0[i] = rr::unpack(raw[0]);
-        if (!p.self_gate) {
-          const float2 g = rr::unpack(raw[1]);
-          e1[i] = make_float2(g.x * rr::sigmoid_fast(g.x), g.y * rr::sigmoid_fast(g.y));
-        }
-      } else {
-        float2 g = rr::unpack(raw[0]);
-        const float2 dy = rr::unpack(raw[1]), h = rr::unpack(raw[2]), v = rr::unpack(raw[3]);
-        if (p.self_gate) g = h;
-        const float sx = rr::sigmoid_fast(g.x), sy = rr::sigmoid_fast(g.y);
-        const float gx = dy.x * h.x * sx * (1.f + g.x * (1.f - sx));
-        const float gy = dy.y * h.y * sy * (1.f + g.y * (1.f - sy));
-        late[i] = rr::pack(gx, gy);
-        e0[i] = make_float2(dy.x * g.x * sx, dy.y * g.y * sy);
-        if (p.self_gate) { e0[i].x += gx; e0[i].y += gy; }   // d(h silu(h))/dh = silu(h) + h silu'(h)
-        e1[i] = make_float2(rr::dtanh_from_v(v.x), rr::dtanh_from_v(v.y));
-      }
-      // computed now, not sunk to their use behind the wait
-      asm volatile("" : "+f"(e0[i].x), "+f"(e0[i].y), "+f"(e1[i].x), "+f"(e1[i].y));
-      if (BWD) asm volatile("" : "+r"(late[i]));
-    }
-  };
-  float2 dbs[ITEMS];
-#pragma unroll
-  for (int i = 0; i < ITEMS; ++i) dbs[i] = make_float2(0.f, 0.f);
-
-#pragma unroll
-  for (int s = 0; s < RR_AHEAD - 1; ++s) fetch(s, at + s * step_bytes);
+  for (int s = 0; s < RR_AHEAD - 1; ++s) tail.fetch(s, at + s * step_bytes);
   const int stall_step = blockIdx.x == 0 ? p.stall_step : -1;
-  int bad = 0;
   uint32_t met = rr::cycles();      // when this CTA's partial sums last met
   __syncthreads();
 
   for (int s = 0; s < T; ++s, at += step_bytes) {
     // ---- the step-local part of this step's arithmetic, then my K range of the group's state:
     // straight into fragments, until all of it is there ----
-    fetch(s + RR_AHEAD - 1, at + (RR_AHEAD - 1) * step_bytes);
-    premath(s);
+    tail.fetch(s + RR_AHEAD - 1, at + (RR_AHEAD - 1) * step_bytes);
+    tail.premath(s);
     const char* src = reinterpret_cast<const char*>(p.state) + (BWD ? at + slot : at);
     while (rr::cycles() - met < (uint32_t)p.hold) { }
     uint4 x[NT][KB];
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int kb = 0; kb < KB; ++kb) x[nt][kb] = rr::ld_relaxed_v4(src + x_off[nt] + kb * 64);
-    if (s > 0) {     // the first slot was written before the launch, whatever it holds
-      long spins = 0;
-      unsigned long long t_begin = 0;
-      while (true) {
-        // one comparison for everything: the pattern is the largest unsigned value
-        uint32_t top = s == stall_step ? 0xFFFFFFFFu : 0u;
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-          for (int kb = 0; kb < KB; ++kb) top = max(top, rr::largest(x[nt][kb]));
-        if (top != 0xFFFFFFFFu) break;
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-          for (int kb = 0; kb < KB; ++kb)
-            if (rr::largest(x[nt][kb]) == 0xFFFFFFFFu)
-              x[nt][kb] = rr::ld_relaxed_v4(src + x_off[nt] + kb * 64);
-        ++spins;
-        bool stop = spins > p.spin_limit;
-        if ((spins & 63) == 0) {
-          const unsigned long long now = ptx::globaltimer_ns();
-          if (t_begin == 0) t_begin = now;
-          stop = stop || ld_relaxed_gpu(p.abort_word) != 0 || now - t_begin > ptx::kWaitDeadlineNs;
-        }
-        if (stop) {
-          if (atomicExch(p.abort_word, 1) == 0)
-            report_timeout(p.status, BWD ? KID_REC_TC_BWD : KID_REC_TC_FWD, s);
-          s_bad[s & 1] = 1;
-          break;
-        }
-      }
+    rr::look(x, src, x_off);
+    // (the first slot was written before the launch, whatever it holds)
+    if (s > 0 && !rr::await(x, src, x_off, s == stall_step, p.spin_limit, p.abort_word)) {
+      if (atomicExch(p.abort_word, 1) == 0)
+        report_timeout(p.status, BWD ? KID_REC_TC_BWD : KID_REC_TC_FWD, s);
+      s_bad[s & 1] = 1;
     }
     __syncwarp();
     float acc[CH][MT][NT][4];
-#pragma unroll
-    for (int ch = 0; ch < CH; ++ch)
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-          for (int u = 0; u < 4; ++u) acc[ch][mt][nt][u] = 0.f;
-#pragma unroll
-    for (int kb = 0; kb < KB; ++kb) {
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-          rr::mma_bf16(acc[0][mt][nt], w[mt][kb][0], w[mt][kb][1], w[mt][kb][2], w[mt][kb][3],
-                       x[nt][kb].x, x[nt][kb].y);
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-          rr::mma_bf16(acc[CH - 1][mt][nt], w[mt][kb][4], w[mt][kb][5], w[mt][kb][6], w[mt][kb][7],
-                       x[nt][kb].z, x[nt][kb].w);
-    }
+    rr::products(acc, w, x);
     // ---- partial sums of the eight K ranges meet in shared memory (two buffers: the barrier of
     // the next step separates this buffer's readers from its next writers) ----
     float* buf = part + (s & 1) * (RR_WARPS * NG * PS);
-    {
-      float* mybuf = buf + (warp * NG + 2 * tq) * PS + gq;
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            float v = acc[0][mt][nt][u];
-            if (CH == 2) v += acc[1][mt][nt][u];
-            mybuf[(nt * 8 + (u & 1)) * PS + mt * 16 + 8 * (u >> 1)] = v;
-          }
-    }
+    rr::put_partials(buf + warp * NG * PS, PS, gq, tq, acc);
     __syncthreads();
     met = rr::cycles();
-
-    bad = s_bad[s & 1];
-    uint32_t o0[ITEMS], o1[ITEMS];
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-      if (!mine[i]) continue;
-      float2 a = BWD ? make_float2(0.f, 0.f) : e0[i];
-      float2 q[RR_WARPS];
-#pragma unroll
-      for (int wv = 0; wv < RR_WARPS; ++wv)
-        q[wv] = *reinterpret_cast<const float2*>(buf + wv * (NG * PS) + spart[i]);
-#pragma unroll
-      for (int st = 1; st < RR_WARPS; st *= 2)
-#pragma unroll
-        for (int wv = 0; wv < RR_WARPS; wv += 2 * st) { q[wv].x += q[wv + st].x; q[wv].y += q[wv + st].y; }
-      a.x += q[0].x; a.y += q[0].y;
-      char* dst = reinterpret_cast<char*>(p.state) + (BWD ? at : at + slot) + off[i];
-      if (!BWD) {
-        const float h0 = rr::tanh_fast(a.x), h1 = rr::tanh_fast(a.y);
-        const uint32_t hp = rr::pack(h0, h1);
-        rr::st_relaxed_u32(dst, hp);
-        o0[i] = rr::pack(a.x, a.y);
-        if (p.self_gate) {     // the gate is the state as stored
-          const float2 hs = rr::unpack(hp);
-          o1[i] = rr::pack(h0 * hs.x * rr::sigmoid_fast(hs.x), h1 * hs.y * rr::sigmoid_fast(hs.y));
-        } else {
-          o1[i] = rr::pack(h0 * e1[i].x, h1 * e1[i].y);
-        }
-      } else {
-        const float d0 = (e0[i].x + a.x) * e1[i].x, d1 = (e0[i].y + a.y) * e1[i].y;
-        rr::st_relaxed_u32(dst, rr::pack(d0, d1));
-        dbs[i].x += d0; dbs[i].y += d1;
-        o0[i] = late[i];
-      }
-    }
-    // ---- outputs that no other CTA waits for ----
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-      if (!mine[i]) continue;
-      if (p.out0 != nullptr) *const_cast<unsigned int*>(word(p.out0, at, off[i])) = o0[i];
-      if (!BWD) *const_cast<unsigned int*>(word(p.out1, at, off[i])) = o1[i];
-    }
+    const int bad = s_bad[s & 1];
+    tail.publish(buf, at);
+    tail.store_rest(at);
     if (bad) break;
   }
-
-  if (BWD) {   // bias gradient: this group's rows of a feature, in a fixed order
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-      const int e = tid + i * RR_THREADS, n = e / PAIRS;
-      if (e < PAIRS * NG) *reinterpret_cast<float2*>(part + n * PS + 2 * (e - n * PAIRS)) = dbs[i];
-    }
-    __syncthreads();
-    if (tid < R && f0 + tid < d) {
-      float sum = 0.f;
-#pragma unroll
-      for (int n = 0; n < NG; ++n) sum += part[n * PS + tid];
-      p.db[(long)grp * d + f0 + tid] = sum;
-    }
-  }
+  if (BWD) tail.fold_bias(part, f0, p.b_lo / NG + grp);
 }
 
 }  // namespace elman

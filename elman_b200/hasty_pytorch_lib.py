@@ -320,8 +320,10 @@ def stock_elman_backward(W_x, W_h, W_gate, x, h, v, gate_cache, d_output):
 
 # --------------------------------------------------------------------------- E5
 
-def pure_lowrank_elman_forward(training, x, h0, U_h, V_h, U_x, V_x, U_z, V_z, b):
-    """-> [h, output, v]"""
+def pure_lowrank_elman_forward(training, x, h0, U_h, V_h, U_x, V_x, U_z, V_z, b, flags=0):
+    """-> [h, output, v]
+
+    `flags` is not a reference argument (see elman_e5_forward_flags)."""
     fn = "pure_lowrank_elman_forward"
     dt = _check_inputs(fn, x, x=x, h0=h0, U_h=U_h, V_h=V_h, U_x=U_x, V_x=V_x, U_z=U_z, V_z=V_z,
                        b=b)
@@ -340,7 +342,8 @@ def pure_lowrank_elman_forward(training, x, h0, U_h, V_h, U_x, V_x, U_z, V_z, b)
         out = torch.empty(T, B, d, dtype=x.dtype, device=x.device)
         v = torch.empty((T, B, d) if training else (0,), dtype=x.dtype, device=x.device)
         ws = _workspace(lib.elman_e5_forward_workspace(dt, T, B, d, r), x.device)
-        rc = lib.elman_e5_forward(dt, 1 if training else 0, T, B, d, r, _ptr(x), _ptr(h0),
+        rc = lib.elman_e5_forward_flags(dt, int(flags), 1 if training else 0, T, B, d, r, _ptr(x),
+                                        _ptr(h0),
                                   _ptr(U_h), _ptr(V_h), _ptr(U_x), _ptr(V_x), _ptr(U_z), _ptr(V_z),
                                   _ptr(b), _ptr(h), _ptr(out), _ptr(v), ws.data_ptr(), ws.numel(),
                                   _stream(x.device))
@@ -375,7 +378,8 @@ def pure_lowrank_elman_backward(U_h, V_h, U_x, V_x, U_z, V_z, x, h, v, d_output)
     return [dx, dU[0], dV[0], dU[1], dV[1], dU[2], dV[2], db]
 
 
-def pure_lowrank_elman_backward_carry(U_h, V_h, U_x, V_x, U_z, V_z, x, h, v, d_output, dv_in=None):
+def pure_lowrank_elman_backward_carry(U_h, V_h, U_x, V_x, U_z, V_z, x, h, v, d_output, dv_in=None,
+                                      flags=0):
     """Backward over one time chunk -> [dx, dU_h, dV_h, dU_x, dV_x, dU_z, dV_z, db, dv_out]
     (an extension, as mamba_gated_elman_backward_carry)."""
     fn = "pure_lowrank_elman_backward_carry"
@@ -398,7 +402,8 @@ def pure_lowrank_elman_backward_carry(U_h, V_h, U_x, V_x, U_z, V_z, x, h, v, d_o
         db = torch.empty(d, dtype=x.dtype, device=x.device)
         dv_out = torch.empty(B, d, dtype=x.dtype, device=x.device)
         ws = _workspace(lib.elman_e5_backward_workspace(dt, T, B, d, r), x.device)
-        rc = lib.elman_e5_backward_carry(dt, T, B, d, r, _ptr(U_h), _ptr(V_h), _ptr(U_x), _ptr(V_x),
+        rc = lib.elman_e5_backward_carry_flags(dt, int(flags), T, B, d, r, _ptr(U_h), _ptr(V_h),
+                                               _ptr(U_x), _ptr(V_x),
                                          _ptr(U_z), _ptr(V_z), _ptr(x), _ptr(h), _ptr(v),
                                          _ptr(d_output), _ptr(dv_in), _ptr(dx), _ptr(dU[0]),
                                          _ptr(dV[0]), _ptr(dU[1]), _ptr(dV[1]), _ptr(dU[2]),

@@ -42,9 +42,10 @@ class PureLowRankElmanChunkFunction(torch.autograd.Function):
     pre-activation gradient of the later chunk's first step backward, not dL/dh."""
 
     @staticmethod
-    def forward(ctx, x, h0, U_h, V_h, U_x, V_x, U_z, V_z, b):
+    def forward(ctx, x, h0, U_h, V_h, U_x, V_x, U_z, V_z, b, flags=0):
+        ctx.kw = {"flags": flags} if flags else {}   # launches that overlap others: smallest footprint
         h, output, v = hasty_pytorch_lib.pure_lowrank_elman_forward(
-            True, x, h0, U_h, V_h, U_x, V_x, U_z, V_z, b)
+            True, x, h0, U_h, V_h, U_x, V_x, U_z, V_z, b, **ctx.kw)
         ctx.save_for_backward(U_h, V_h, U_x, V_x, U_z, V_z, x, h, v)
         ctx.set_materialize_grads(False)
         return output, h[-1].clone()
@@ -61,9 +62,9 @@ class PureLowRankElmanChunkFunction(torch.autograd.Function):
                 dv_in.record_stream(here)
         r = hasty_pytorch_lib.pure_lowrank_elman_backward_carry(
             U_h, V_h, U_x, V_x, U_z, V_z, x, h, v, grad_output.contiguous(),
-            None if dv_in is None else dv_in.contiguous())
+            None if dv_in is None else dv_in.contiguous(), **ctx.kw)
         dx, dU_h, dV_h, dU_x, dV_x, dU_z, dV_z, db, dv_out = r
-        return dx, dv_out, dU_h, dV_h, dU_x, dV_x, dU_z, dV_z, db
+        return dx, dv_out, dU_h, dV_h, dU_x, dV_x, dU_z, dV_z, db, None
 
 
 class PureLowRankElmanCell(nn.Module):
@@ -135,7 +136,7 @@ class PureLowRankElman(nn.Module):
         c = self.cell
         return PureLowRankElmanChunkFunction.apply(
             pre, h0.contiguous(), c.U_h.contiguous(), c.V_h.contiguous(), c.U_x.contiguous(),
-            c.V_x.contiguous(), c.U_z.contiguous(), c.V_z.contiguous(), c.b.contiguous())
+            c.V_x.contiguous(), c.U_z.contiguous(), c.V_z.contiguous(), c.b.contiguous(), flags)
 
     def chunk_post(self, cell_out):
         return self.dropout(cell_out)

@@ -382,7 +382,23 @@ int elman_e5_backward_carry(int dtype, int T, int B, int d, int r,
                             void* dU_z, void* dV_z, void* db,
                             void* dv_out,
                             void* workspace, size_t workspace_bytes, void* stream);
-/* Thread blocks an E5 recurrence launch of this shape keeps resident (one cluster), or 0
+/* The same with flags (ELMAN_FLAG_COMPACT: the single-cluster kernel where it takes the shape,
+ * for callers that overlap several recurrence launches). */
+int elman_e5_forward_flags(int dtype, int flags, int training, int T, int B, int d, int r,
+                           const void* x, const void* h0,
+                           const void* U_h, const void* V_h, const void* U_x, const void* V_x,
+                           const void* U_z, const void* V_z, const void* b,
+                           void* h, void* output, void* v,
+                           void* workspace, size_t workspace_bytes, void* stream);
+int elman_e5_backward_carry_flags(int dtype, int flags, int T, int B, int d, int r,
+                                  const void* U_h, const void* V_h, const void* U_x,
+                                  const void* V_x, const void* U_z, const void* V_z,
+                                  const void* x, const void* h, const void* v,
+                                  const void* d_output, const void* dv_in,
+                                  void* dx, void* dU_h, void* dV_h, void* dU_x, void* dV_x,
+                                  void* dU_z, void* dV_z, void* db, void* dv_out,
+                                  void* workspace, size_t workspace_bytes, void* stream);
+/* Thread blocks an E5 recurrence launch (ELMAN_FLAG_COMPACT) of this shape keeps resident (one cluster), or 0
  * when the shape takes the cooperative-launch kernel; see elman_b200_recurrence_blocks. */
 int elman_b200_lowrank_blocks(int dtype, int T, int B, int d, int r);
 
