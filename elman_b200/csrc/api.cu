@@ -167,8 +167,9 @@ static size_t splitk_scratch_bytes(int dtype, int M, int N) {
 static int gemm_tn(int dtype, int M, int N, long K, const void* Am, const void* Bm, void* C,
                    cudaStream_t st, float* splitk, size_t splitk_bytes, int accumulate) {
   if (M == 0 || N == 0) return ELMAN_OK;
-  if (use_tc(dtype) && K < (1L << 31) && (M & 7) == 0 && (N & 7) == 0 && (K & 7) == 0 &&
-      gemm_tc_supported(M, N, (int)K, Am, M, Bm, N, C, N, 0)) {
+  // (K counts rows of both operands, so no alignment rule touches it: a tail is zero-filled)
+  if (use_tc(dtype) && K > 0 && K < (1L << 31) && (M & 7) == 0 && (N & 7) == 0 &&
+      gemm_tc_supported(M, N, 8, Am, M, Bm, N, C, N, 0)) {
     return gemm_tc(M, N, (int)K, (const bf16*)Am, M, 1, (const bf16*)Bm, N, 1, nullptr, C, N, 0,
                    accumulate, st, splitk, splitk_bytes);
   }

@@ -1231,7 +1231,7 @@ int gemm_tc_pair(int M, int N, int K, const bf16* A, int lda, int a_mn, const bf
 int gemm_tc_dual_tn(int M, int N, int K, const bf16* A, const bf16* B1, const bf16* B2, void* C1,
                     void* C2, cudaStream_t stream) {
   if (options().gemm_pair == 1 || M < Q_BM || N < Q_BN || (M & 7) != 0 || (N & 7) != 0 ||
-      (K & 7) != 0 || !gemm_tc_supported(M, N, K, A, M, B1, N, C1, N, 0))
+      K < 1 || !gemm_tc_supported(M, N, 8, A, M, B1, N, C1, N, 0))
     return ELMAN_ERR_UNSUPPORTED;
   GemmParams q;
   q.M = M; q.N = N; q.K = K;
