@@ -259,6 +259,10 @@ static int run_rec_fwd(int dtype, int T, int B, int d, const void* W, const void
     const int rc = rec_fwd_tc(a, st);
     if (rc != ELMAN_ERR_UNSUPPORTED) return rc;
   }
+  if (dtype == ELMAN_F32 && rec_f32_supported(T, B, d)) {
+    const int rc = rec_fwd_f32(a, st);
+    if (rc != ELMAN_ERR_UNSUPPORTED) return rc;
+  }
   return rec_fwd_generic(dtype, a, st);
 }
 
@@ -285,6 +289,10 @@ static int run_rec_bwd(int dtype, int T, int B, int d, const void* Wt, const voi
   if (dense_tc_ok(dtype, T, B, d, 1)) {
     const int rc = rec_bwd_tc(a, st);
     if (rc != ELMAN_ERR_UNSUPPORTED) return rc;   // see run_rec_fwd
+  }
+  if (dtype == ELMAN_F32 && rec_f32_supported(T, B, d)) {
+    const int rc = rec_bwd_f32(a, st);
+    if (rc != ELMAN_ERR_UNSUPPORTED) return rc;
   }
   return rec_bwd_generic(dtype, a, st);
 }

@@ -121,6 +121,10 @@ int gemm_generic(int dtype, int M, int N, int K, const void* A, long sAm, long s
                  const void* B, long sBk, long sBn, const void* bias, void* C, long ldc,
                  int accumulate, cudaStream_t stream);
 
+// The fp32 form (gemm_f32.cu); ELMAN_ERR_UNSUPPORTED when an operand has no unit stride.
+int gemm_f32(int M, int N, int K, const float* A, long sAm, long sAk, const float* B, long sBk, long sBn,
+             const float* bias, float* C, long ldc, int accumulate, cudaStream_t stream);
+
 // C[M,N] = A[M,K] * W[N,K]^T, bf16, TMA + tcgen05.  Returns ELMAN_ERR_UNSUPPORTED
 // (without setting an error message) when the shape or alignment rules it out.
 int gemm_tc_nt(int M, int N, int K, const bf16* A, int lda, const bf16* W, int ldw,
@@ -263,6 +267,10 @@ bool rec_reg_supported(int T, int B, int d);
 int rec_reg_blocks(int B, int d);
 int rec_fwd_reg(const RecFwdArgs& a, cudaStream_t stream);
 int rec_bwd_reg(const RecBwdArgs& a, cudaStream_t stream);
+// Dense recurrence, fp32, W in registers (rec_f32.cu).
+bool rec_f32_supported(int T, int B, int d);
+int rec_fwd_f32(const RecFwdArgs& a, cudaStream_t stream);
+int rec_bwd_f32(const RecBwdArgs& a, cudaStream_t stream);
 int rec_reg_sms();   // multiprocessors of the current device
 
 // Low-rank recurrence, bf16, both factors in registers (lowrank_reg.cuh): d % 8 == 0, d from 64 to

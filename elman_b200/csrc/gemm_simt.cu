@@ -137,6 +137,11 @@ int gemm_generic(int dtype, int M, int N, int K, const void* A, long sAm, long s
                  const void* B, long sBk, long sBn, const void* bias, void* C, long ldc,
                  int accumulate, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return ELMAN_OK;
+  if (dtype == ELMAN_F32) {
+    const int rc = gemm_f32(M, N, K, (const float*)A, sAm, sAk, (const float*)B, sBk, sBn,
+                            (const float*)bias, (float*)C, ldc, accumulate, stream);
+    if (rc != ELMAN_ERR_UNSUPPORTED) return rc;
+  }
   dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM);
   if (dtype == ELMAN_F32) {
     gemm_simt_kernel<float><<<grid, 256, 0, stream>>>(
