@@ -15,6 +15,7 @@ LIB_PATH = os.path.join(_HERE, "lib", "libelman_b200.so")
 HEADER_PATH = os.path.join(_HERE, "..", "include", "elman_b200.h")
 
 ELMAN_OK = 0
+ELMAN_ERR_UNSUPPORTED = 5
 ELMAN_F32 = 0
 ELMAN_BF16 = 1
 
@@ -84,6 +85,9 @@ SIGNATURES = {
     "elman_e33_forward": (_I, [_I, _I, _I, _I, _I] + [_P] * 5 + [_P] * 3 + [_P, _Z, _P]),
     "elman_e33_backward_workspace": (_Z, [_I, _I, _I, _I]),
     "elman_e33_backward": (_I, [_I, _I, _I, _I] + [_P] * 6 + [_P] * 4 + [_P, _Z, _P]),
+    "elman_e1_lm_token_supported": (_I, [_I] * 5),
+    "elman_e1_lm_token_workspace": (_Z, [_I] * 3),
+    "elman_e1_lm_token": (_I, [_I] * 5 + [_P] * 5 + [_F] * 3 + [_P, _P, _Z, _P]),
     "elman_adamw_step": (_I, [_I, _L, _P, _P, _P, _P] + [_c.c_float] * 5 + [_P, _P, _P]),
     "elman_projection": (_I, [_I, _I, _I, _I, _P, _I, _P, _I, _P, _P, _I, _I, _P]),
 }

@@ -45,19 +45,29 @@ def _library_takes(W_h: torch.Tensor) -> bool:
             and W_h.dtype in (torch.float32, torch.bfloat16))
 
 
-def spectrally_normalised(module, W_h: torch.Tensor) -> torch.Tensor:
-    dim = W_h.shape[0]
+def _start_vector(module, W_h):
     u = getattr(module, "_spectral_u", None)
-    if u is None or u.shape[0] != dim:
-        u = torch.randn(dim, device=W_h.device, dtype=W_h.dtype)
+    if u is None or u.shape[0] != W_h.shape[0]:
+        u = torch.randn(W_h.shape[0], device=W_h.device, dtype=W_h.dtype)
         u = u / u.norm()
-    if _library_takes(W_h):
-        # keep the vector in place once it exists: a captured CUDA graph then reads and
-        # advances the same buffer on every replay
-        if u.device != W_h.device or u.dtype != W_h.dtype or not u.is_contiguous():
-            u = u.to(device=W_h.device, dtype=W_h.dtype).contiguous()
+    return u
+
+
+def library_vector(module, W_h: torch.Tensor) -> torch.Tensor:
+    """The persistent vector of `module`, where and how the library's kernels advance it in place: a
+    captured CUDA graph then reads and advances the same buffer on every replay."""
+    u = module.__dict__.get("_spectral_u")
+    if u is None or u.device != W_h.device or u.dtype != W_h.dtype or u.shape[0] != W_h.shape[0] \
+            or not u.is_contiguous():
+        u = _start_vector(module, W_h).to(device=W_h.device, dtype=W_h.dtype).contiguous()
         module._spectral_u = u
-        return SpectralNormFunction.apply(W_h, u)
+    return u
+
+
+def spectrally_normalised(module, W_h: torch.Tensor) -> torch.Tensor:
+    if _library_takes(W_h):
+        return SpectralNormFunction.apply(W_h, library_vector(module, W_h))
+    u = _start_vector(module, W_h)
     with torch.no_grad():
         for _ in range(POWER_ITERS):
             v = W_h.T @ u

@@ -1623,6 +1623,34 @@ int elman_silu_backward_concat(int dtype, long M, int d_inner, const void* d_act
   return silu_bwd_concat(dtype, M, d_inner, d_act, x_raw, dz, dxz, (cudaStream_t)stream);
 }
 
+int elman_e1_lm_token_supported(int dtype, int depth, int B, int d, int vocab) {
+  return lm_token_supported(dtype, depth, B, d, vocab) ? 1 : 0;
+}
+
+size_t elman_e1_lm_token_workspace(int depth, int B, int d) {
+  return lm_token_workspace(depth < 1 ? 1 : depth, B < 1 ? 1 : B, d);
+}
+
+int elman_e1_lm_token(int dtype, int depth, int B, int d, int vocab, const long long* tokens,
+                      const void* embedding, const void* const* layers, const void* norm,
+                      const void* head, float eps, float target_radius, float spectral_eps,
+                      void* logits, void* workspace, size_t workspace_bytes, void* stream) {
+  ELMAN_RETURN_IF(check_common(dtype, 1, B, d));
+  if (!lm_token_supported(dtype, depth, B, d, vocab))
+    return set_error(ELMAN_ERR_UNSUPPORTED, "depth %d, B %d, d %d: not a shape of elman_e1_lm_token", depth, B, d);
+  REQUIRE_PTR(tokens); REQUIRE_PTR(embedding); REQUIRE_PTR(layers); REQUIRE_PTR(norm); REQUIRE_PTR(head);
+  REQUIRE_PTR(logits); REQUIRE_PTR(workspace);
+  ELMAN_ARG_CHECK(((uintptr_t)workspace & 255) == 0, "workspace must be 256-byte aligned");
+  const size_t need = lm_token_workspace(depth, B, d);
+  if (workspace_bytes < need)
+    return set_error(ELMAN_ERR_WORKSPACE, "workspace %zu < required %zu", workspace_bytes, need);
+  LmTokenArgs a{depth, B, d, vocab, tokens, embedding, layers, norm, head, eps, target_radius,
+                spectral_eps, logits, workspace};
+  const int rc = lm_token(a, (cudaStream_t)stream);
+  if (rc == ELMAN_ERR_UNSUPPORTED) return set_error(rc, "an operand is not 16-byte aligned");
+  return rc;
+}
+
 int elman_adamw_step(int dtype, long n, void* params, const void* grads, void* exp_avg,
                      void* exp_avg_sq, float lr, float beta1, float beta2, float eps,
                      float weight_decay, float* step, const float* grad_scale, void* stream) {

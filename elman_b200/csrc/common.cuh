@@ -71,7 +71,7 @@ int* device_status_ptr();   // device-side alias, or nullptr if unavailable
 
 // kernel ids recorded in the status word
 enum KernelId { KID_REC_SIMT = 1, KID_REC_TC_FWD = 2, KID_REC_TC_BWD = 3, KID_GEMM_TC = 4,
-                KID_LOWRANK_SIMT = 5, KID_WAIT_PROBE = 6, KID_LOWRANK_TC = 7 };
+                KID_LOWRANK_SIMT = 5, KID_WAIT_PROBE = 6, KID_LOWRANK_TC = 7, KID_LM_TOKEN = 8 };
 
 // ---------------------------------------------------------------------------
 // device helpers
@@ -292,6 +292,25 @@ struct LowRankRegArgs {
 };
 bool lowrank_reg_supported(int T, int B, int d, int r);
 int lowrank_reg(const LowRankRegArgs& a, cudaStream_t stream);
+
+// One token through a stack of E1 layers, final norm and head (lm_token.cu).  Pointers per layer:
+// norm, in_proj, W_x, W_h, b, out_proj, u (spectral norm's vector, advanced in place; null: none),
+// h_prev (null: zeros), h_out.
+constexpr int LM_TOKEN_REFS = 9;
+struct LmTokenArgs {
+  int L, B, d, V;
+  const long long* tokens;       // [B]
+  const void* embedding;         // [V, d]
+  const void* const* layers;     // [L][LM_TOKEN_REFS]
+  const void* norm;              // [d]
+  const void* head;              // [V, d]
+  float eps, target, spectral_eps;
+  void* logits;                  // [B, V]
+  void* workspace;
+};
+bool lm_token_supported(int dtype, int L, int B, int d, int V);
+size_t lm_token_workspace(int L, int B, int d);
+int lm_token(const LmTokenArgs& a, cudaStream_t stream);
 
 // Copies the cycle stamps of the last traced launch (option rec_trace) to the host.
 int rec_tc_copy_trace(long long* dst, int max_entries);

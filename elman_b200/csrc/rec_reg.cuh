@@ -157,7 +157,7 @@ __device__ __forceinline__ bool await(uint4 (&x)[NT][KB], const char* src, const
     if ((spins & 63) == 0) {
       const unsigned long long now = ptx::globaltimer_ns();
       if (t_begin == 0) t_begin = now;
-      if (ld_relaxed_gpu(abort_word) != 0 || now - t_begin > ptx::kWaitDeadlineNs) return false;
+      if (ld_relaxed_gpu(abort_word) == 1 || now - t_begin > ptx::kWaitDeadlineNs) return false;
     }
   }
 }

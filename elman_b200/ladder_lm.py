@@ -9,15 +9,20 @@ residual stream -> Elman layer) -> final add + norm -> tied linear head ->
 arguments that only concern other levels of the reference are accepted and
 ignored.
 """
+import contextlib
+import ctypes
+
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from . import fused_ops
+from . import _lib, _spectral, fused_ops
 from .mamba_gated_elman import MambaGatedElman
 from .pure_lowrank_elman import PureLowRankElman
 from .siblings import E32NoPresilu, E33SelfGate, E57LearnedRadius, LowRankElman
 from .stock_elman import StockElman
+
+_NO_SWITCH = contextlib.nullcontext()
 
 _LEVELS = {0: StockElman, 1: MambaGatedElman, 4: LowRankElman, 5: PureLowRankElman,
            32: E32NoPresilu, 33: E33SelfGate, 57: E57LearnedRadius}
@@ -81,6 +86,10 @@ class LadderLM(nn.Module):
             inp = x
         if prev_hiddens is None:
             prev_hiddens = [None] * self.depth
+        if not return_loss and inp.size(1) == 1 and not torch.is_grad_enabled():
+            token = self._one_token(inp, prev_hiddens)
+            if token is not None:
+                return (token[0], (token[1], None)) if return_prev_hiddens else token[0]
         sink = fused_ops.get_grad_sink()
         if sink is not None and torch.is_grad_enabled():
             sink.begin_pass()
@@ -143,6 +152,96 @@ class LadderLM(nn.Module):
             loss = F.cross_entropy(self._head(h).view(-1, self.vocab_size), target.reshape(-1),
                                    ignore_index=-100)
         return (loss, (new_hiddens, None)) if return_prev_hiddens else loss
+
+    def _one_token(self, inp, prev_hiddens):
+        """One more token for every sequence (inp [B,1], no gradients) through the whole stack in the
+        library's generation kernel: (logits [B,1,V], [final state of every layer]) — or None
+        when the model or the tensors are not what that kernel takes.
+
+        Issuing the step must not take longer than the step.  The parameters are looked up anew on
+        every call, by the shortest way (dictionaries instead of nn.Module attribute access); what
+        follows from them alone is checked again only when one of their addresses or types is not
+        the one it was."""
+        mods = self._modules
+        emb = mods["embedding"]._parameters["weight"]
+        dtype, d = emb.dtype, self.dim
+        if dtype is not torch.bfloat16 or not emb.is_cuda or not self.fused_ops \
+                or inp.dtype is not torch.int64 or not inp.is_cuda:
+            return None
+        params, addresses = [emb], []
+        vectors, eps = [], [mods["norm"].eps]
+        for layer, ln in zip(mods["layers"]._modules.values(), mods["layer_norms"]._modules.values()):
+            lm = layer._modules
+            cell = lm.get("cell")
+            if type(layer) is not MambaGatedElman or layer.use_conv or not layer.fused \
+                    or layer.d_inner != d or (self.training and type(lm["dropout"]) is nn.Dropout):
+                return None
+            cp = cell._parameters
+            W_h = cp["W_h"]
+            params += (ln._parameters["weight"], lm["in_proj"]._parameters["weight"], cp["W_x"], W_h,
+                       cp["b"], lm["out_proj"]._parameters["weight"])
+            eps.append(ln.eps)
+            vectors.append(_spectral.library_vector(cell, W_h)
+                           if cell.w_h_mode == "spectral_norm" and W_h.is_cuda else None)
+        params += (mods["norm"]._parameters["weight"], mods["lm_head"]._parameters["weight"])
+        if not _spectral.FUSED:
+            return None
+        addresses = [(p.data_ptr(), p.dtype) for p in params] + eps
+        plan = self.__dict__.get("_token_plan")
+        if plan is None or plan[0] != addresses:
+            plan = self.__dict__["_token_plan"] = (addresses, *self._token_plan_for(params))
+        _, table0, device, eps = plan
+        if table0 is None or inp.device != device:
+            return None
+        B, depth, V = inp.size(0), self.depth, self.vocab_size
+        lib = _lib.load()
+        if not lib.elman_e1_lm_token_supported(_lib.ELMAN_BF16, depth, B, d, V):
+            return None
+        table = type(table0).from_buffer_copy(table0)
+        hiddens = torch.empty(depth, B, d, dtype=dtype, device=device)
+        h_out, h_bytes, shape = hiddens.data_ptr(), B * d * 2, (B, d)
+        keep = []
+        for i, (h, u) in enumerate(zip(prev_hiddens, vectors)):
+            at = 9 * i + 6
+            if u is not None:
+                table[at] = u.data_ptr()
+            if h is not None:
+                if h.dtype is not dtype or h.device != device or h.shape != shape:
+                    return None
+                if not h.is_contiguous():
+                    h = h.contiguous()
+                    keep.append(h)
+                table[at + 1] = h.data_ptr()
+            table[at + 2] = h_out + i * h_bytes
+        tokens = inp.contiguous()
+        logits = torch.empty(B, 1, V, dtype=dtype, device=device)
+        with torch.cuda.device(device) if torch.cuda.current_device() != device.index else _NO_SWITCH:
+            ws = torch.empty(lib.elman_e1_lm_token_workspace(depth, B, d), dtype=torch.uint8, device=device)
+            rc = lib.elman_e1_lm_token(
+                _lib.ELMAN_BF16, depth, B, d, V, tokens.data_ptr(), addresses[0][0], table,
+                params[-2].data_ptr(), params[-1].data_ptr(), eps, _spectral.TARGET_RADIUS, _spectral.EPS,
+                logits.data_ptr(), ws.data_ptr(), ws.numel(),
+                torch.cuda.current_stream(device).cuda_stream)
+        if rc == _lib.ELMAN_ERR_UNSUPPORTED:     # an operand off its 16-byte boundary
+            return None
+        _lib.check(rc, "elman_e1_lm_token")
+        return logits, list(hiddens.unbind(0))
+
+    def _token_plan_for(self, params):
+        """(pointer table without the per-call entries, device, epsilon) of the generation kernel, or
+        (None, None, None) when it does not take these parameters."""
+        no = (None, None, None)
+        device = params[0].device
+        if any(p.dtype != torch.bfloat16 or p.device != device or not p.is_contiguous() for p in params):
+            return no
+        norms = list(self.layer_norms) + [self.norm]
+        if any(getattr(n, "eps", None) != norms[0].eps for n in norms):
+            return no
+        table = (ctypes.c_void_p * (9 * self.depth))()
+        for i in range(self.depth):
+            for j in range(6):
+                table[9 * i + j] = params[1 + 6 * i + j].data_ptr()
+        return table, device, fused_ops.rmsnorm_eps(self.norm, torch.bfloat16)
 
     def _add_norm(self, norm, h, residual, last=False, group=None):
         """residual = h + residual (fp32 stream); h = norm(residual in the layer's dtype).

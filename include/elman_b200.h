@@ -540,6 +540,23 @@ int elman_adamw_step(int dtype, long n, void* params, const void* grads, void* e
                      void* exp_avg_sq, float lr, float beta1, float beta2, float eps,
                      float weight_decay, float* step, const float* grad_scale, void* stream);
 
+/*
+ * One token for B sequences through `depth` E1 layers with their pre-norms, the final norm and the
+ * head: the generation step of the byte-level model (elman/models/ladder_lm.py:986-1062 with
+ * elman/models/mamba_gated_elman.py:123-146, :283-306), bf16, d_inner = d.  `layers` holds nine
+ * pointers per layer: norm [d], in_proj [2d,d], W_x [d,d], W_h [d,d], b [d], out_proj [d,d],
+ * u [d] (spectral normalisation's vector, advanced in place; NULL: W_h as it is),
+ * h_prev [B,d] (NULL: zeros), h_out [B,d].  Outputs: h_out of every layer, logits [B,vocab].
+ * Matrices, norms, embedding and h_prev must be 16-byte aligned.  A token outside [0, vocab) sets
+ * the device status word (detail 8 << 24 | 0xFFFFFE).
+ */
+int elman_e1_lm_token_supported(int dtype, int depth, int B, int d, int vocab);
+size_t elman_e1_lm_token_workspace(int depth, int B, int d);
+int elman_e1_lm_token(int dtype, int depth, int B, int d, int vocab, const long long* tokens,
+                      const void* embedding, const void* const* layers, const void* norm,
+                      const void* head, float eps, float target_radius, float spectral_eps,
+                      void* logits, void* workspace, size_t workspace_bytes, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

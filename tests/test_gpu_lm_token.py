@@ -1,0 +1,75 @@
+"""LadderLM's generation step in one kernel (csrc/lm_token.cu) against the same model layer by layer, at
+the edges of its tiles: sequences around the 8-row tiles and the 32-row turns, widths that leave a CTA
+or a warp's K range partly filled, with and without carried states, with and without spectral
+normalisation.  Tolerance: the parity tests' bf16 2e-2 — both sides round activations to 8 bits six
+times per layer."""
+import pytest
+import torch
+
+from _gpu_cases import TOL, option
+from elman_b200 import _lib
+from elman_b200.ladder_lm import LadderLM
+from oracle import elman_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def _model(d, depth, mode):
+    torch.manual_seed(d)
+    return LadderLM(vocab_size=256, dim=d, depth=depth, level=1, r_h_mode=mode).cuda().bfloat16().eval()
+
+
+@pytest.mark.parametrize("B,d,depth,mode", [(1, 1280, 3, "spectral_norm"), (8, 40, 2, "none"), (9, 264, 2, "none"),
+                                            (17, 496, 3, "spectral_norm"), (33, 264, 2, "spectral_norm"),
+                                            (64, 1024, 2, "none"), (3, 1368, 2, "spectral_norm")])
+@pytest.mark.parametrize("carried", [True, False])
+def test_one_token_matches_layer_by_layer(B, d, depth, mode, carried):
+    model = _model(d, depth, mode)
+    g = torch.Generator().manual_seed(B)
+    tokens = torch.randint(0, 256, (B, 1), generator=g).cuda()
+    states = [torch.tanh(torch.randn(B, d, generator=g)).bfloat16().cuda() for _ in range(depth)] if carried else None
+    us = [torch.nn.functional.normalize(torch.randn(d, generator=g), dim=0).bfloat16().cuda() for _ in range(depth)]
+    outs = []
+    for off in (1, 0):
+        for layer, u in zip(model.layers, us):
+            layer.cell._spectral_u = u.clone()
+        with torch.no_grad(), option("rec_reg", off):
+            before = _lib.launch_count()
+            logits, (hs, extra) = model(tokens, return_prev_hiddens=True, prev_hiddens=states)
+            launches = _lib.launch_count() - before
+        torch.cuda.synchronize()
+        assert extra is None and logits.shape == (B, 1, 256) and all(h.shape == (B, d) for h in hs)
+        outs.append([logits] + list(hs) + ([l.cell._spectral_u for l in model.layers] if mode != "none" else []))
+    assert launches <= 3, "the generation kernel was not used"
+    assert _lib.device_status()[0] == 0
+    for a, b in zip(outs[1], outs[0]):
+        assert orc.rel_err(a.float().cpu(), b.float().cpu()) < TOL[torch.bfloat16]
+
+
+def test_changed_parameters_are_seen_and_a_token_outside_the_vocabulary_is_reported():
+    model = _model(64, 2, "none")
+    tok = torch.tensor([[3]]).cuda()
+    with torch.no_grad():
+        a = model(tok)
+        model.layers[0].cell.W_x.mul_(0.5)                              # in place
+        b = model(tok)
+        model.layers[1].cell.W_x.data = model.layers[1].cell.W_x * 0.5   # another tensor
+        c = model(tok)
+        assert not torch.equal(a, b) and not torch.equal(b, c)
+        model(torch.tensor([[256]]).cuda())
+        torch.cuda.synchronize()
+    code, detail = _lib.device_status(clear=True)
+    assert code == 3 and detail >> 24 == 8
+
+
+def test_gives_up_when_a_block_stalls_and_recovers():
+    model = _model(64, 3, "none")
+    tok = torch.tensor([[3], [5]]).cuda()
+    with torch.no_grad():
+        want = model(tok)
+        with option("spin_limit", 5000), option("test_stall_step", 1):
+            model(tok)
+        torch.cuda.synchronize()
+        code, detail = _lib.device_status(clear=True)
+        assert code == 3 and detail >> 24 == 8
+        assert torch.equal(model(tok), want)
