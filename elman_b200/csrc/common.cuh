@@ -203,7 +203,7 @@ struct RecFwdArgs {
   void* y;            // [T,B,d]
   void* v;            // [T,B,d] or null
   int* sync;          // zeroed ints (barrier / step counters)
-  int compact = 0;    // tensor-core kernel: prefer the plan with the fewest resident blocks
+  int compact = 0;    // prefer the plan with the fewest resident blocks
 };
 struct RecBwdArgs {
   int T, B, d;
@@ -264,7 +264,7 @@ int rec_bwd_tc(const RecBwdArgs& a, cudaStream_t stream);
 constexpr int RR_MAX_BATCH = 64;
 constexpr int RR_MIN_CONCURRENT_D = 128;
 bool rec_reg_supported(int T, int B, int d);
-int rec_reg_blocks(int B, int d);
+int rec_reg_blocks(int B, int d, int compact);
 int rec_fwd_reg(const RecFwdArgs& a, cudaStream_t stream);
 int rec_bwd_reg(const RecBwdArgs& a, cudaStream_t stream);
 // Dense recurrence, fp32, W in registers (rec_f32.cu).

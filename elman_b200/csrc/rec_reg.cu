@@ -11,7 +11,8 @@ namespace {
 
 struct RecRegPlan {
   int mt, kb, nt;
-  int groups, cpg;
+  int groups, cpg;        // batch groups, or sets of `turns` groups, that have CTAs of their own
+  int turns;              // 0: no turns, rec_reg_kernel
   bool ok;
 };
 
@@ -74,6 +75,32 @@ RecRegPlan pick_rec_reg_plan(int B, int d) {
   return best;
 }
 
+// The plan for callers that overlap launches: the most rows of W per CTA, and as many of the batch
+// groups on one set of CTAs as make the launch a sixth of the device, so that six fit (the pipelined
+// model runs up to one per layer).  Measured, one optimizer step in ms with one set / with two:
+// d 1280 B 32, six layers, 20 / 40 CTAs 11.52 / 11.62; d 768 B 13, six layers, 12 / 24 CTAs 3.32 /
+// 3.23; d 256 B 32, four layers, 4 / 8 CTAs 1.64 / 1.54.  Where every group has its own CTAs this
+// is rec_reg_kernel; a plan with more CTAs than the fast one is of no use.
+RecRegPlan pick_compact_plan(int B, int d) {
+  const RecRegPlan fast = pick_rec_reg_plan(B, d);
+  if (!fast.ok) return fast;
+  RecRegPlan pl = fast;
+  pl.mt = rr::turns_mt(pl.kb);
+  pl.nt = 1;
+  pl.cpg = (d + 16 * pl.mt - 1) / (16 * pl.mt);
+  const int groups = (B + 7) / 8;
+  int sets = rec_reg_sms() / 6 / pl.cpg;
+  sets = sets < 1 ? 1 : sets > groups ? groups : sets;
+  pl.turns = (groups + sets - 1) / sets;
+  pl.groups = (groups + pl.turns - 1) / pl.turns;
+  if (pl.turns == 1) pl.turns = 0;
+  return pl.groups * pl.cpg <= fast.groups * fast.cpg ? pl : fast;
+}
+
+RecRegPlan plan_for(int B, int d, int compact) {
+  return compact ? pick_compact_plan(B, d) : pick_rec_reg_plan(B, d);
+}
+
 // Options that select a plan of the TMEM kernel select that kernel.
 bool rr_enabled() {
   const Options& o = options();
@@ -82,18 +109,22 @@ bool rr_enabled() {
 }
 
 int rr_launch(bool bwd, const RecRegPlan& pl, RecRegParams& p, int* sync, cudaStream_t stream) {
-  RecRegKernel kern = bwd ? rec_reg_bwd_kernel(pl.mt, pl.kb, pl.nt)
-                          : rec_reg_fwd_kernel(pl.mt, pl.kb, pl.nt);
-  // rows of W and of the state are read 16 bytes at a time, the rest in feature pairs
+  const bool turns = pl.turns > 0;
+  RecRegKernel kern = turns ? (bwd ? rec_turns_bwd_kernel(pl.kb) : rec_turns_fwd_kernel(pl.kb))
+                      : bwd ? rec_reg_bwd_kernel(pl.mt, pl.kb, pl.nt)
+                            : rec_reg_fwd_kernel(pl.mt, pl.kb, pl.nt);
+  // rows of W and of the state are read 16 bytes at a time, the rest in feature pairs (turns: fours)
   const uintptr_t wide = (uintptr_t)p.W | (uintptr_t)p.state;
   const uintptr_t narrow = (uintptr_t)p.in0 | (uintptr_t)p.in1 | (uintptr_t)p.in2 | (uintptr_t)p.in3 |
                            (uintptr_t)p.out0 | (uintptr_t)p.out1;
-  if (kern == nullptr || (wide & 15) != 0 || (narrow & 3) != 0) return ELMAN_ERR_UNSUPPORTED;
-  const size_t smem = rec_reg_smem(bwd, pl.mt, pl.nt);
+  if (kern == nullptr || (wide & 15) != 0 || (narrow & (turns ? 7 : 3)) != 0)
+    return ELMAN_ERR_UNSUPPORTED;
+  const size_t smem = turns ? rec_turns_smem(bwd, pl.mt) : rec_reg_smem(bwd, pl.mt, pl.nt);
   if (smem > 48 * 1024)
     ELMAN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   p.b_lo = 0; p.b_hi = p.B;
   p.cpg = pl.cpg;
+  p.turns = pl.turns;
   p.hold = rr_hold(p.B, p.d, pl.cpg);
   p.abort_word = sync;
   p.status = device_status_ptr();
@@ -108,7 +139,7 @@ int rr_launch(bool bwd, const RecRegPlan& pl, RecRegParams& p, int* sync, cudaSt
   // plan for (elman_b200_recurrence_blocks reports 0), ask for it.
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(pl.groups * pl.cpg);
-  cfg.blockDim = dim3(RR_THREADS);
+  cfg.blockDim = dim3(turns ? RR_TURN_THREADS : RR_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr;
@@ -137,13 +168,13 @@ bool rec_reg_supported(int T, int B, int d) {
   return T >= 1 && rr_enabled() && pick_rec_reg_plan(B, d).ok;
 }
 
-int rec_reg_blocks(int B, int d) {
-  const RecRegPlan pl = pick_rec_reg_plan(B, d);
+int rec_reg_blocks(int B, int d, int compact) {
+  const RecRegPlan pl = plan_for(B, d, compact);
   return pl.ok && d >= RR_MIN_CONCURRENT_D ? pl.groups * pl.cpg : 0;
 }
 
 int rec_fwd_reg(const RecFwdArgs& a, cudaStream_t stream) {
-  const RecRegPlan pl = pick_rec_reg_plan(a.B, a.d);
+  const RecRegPlan pl = plan_for(a.B, a.d, a.compact);
   if (!pl.ok) return ELMAN_ERR_UNSUPPORTED;
   RecRegParams p{};
   p.T = a.T; p.B = a.B; p.d = a.d;
@@ -155,7 +186,7 @@ int rec_fwd_reg(const RecFwdArgs& a, cudaStream_t stream) {
 }
 
 int rec_bwd_reg(const RecBwdArgs& a, cudaStream_t stream) {
-  const RecRegPlan pl = pick_rec_reg_plan(a.B, a.d);
+  const RecRegPlan pl = plan_for(a.B, a.d, a.compact);
   if (!pl.ok) return ELMAN_ERR_UNSUPPORTED;
   RecRegParams p{};
   p.T = a.T; p.B = a.B; p.d = a.d;

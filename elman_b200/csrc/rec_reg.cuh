@@ -57,7 +57,8 @@ inline size_t rec_reg_smem(bool bwd, int mt, int nt) {
 struct RecRegParams {
   int T, B, d;
   int b_lo, b_hi;         // batch rows of this launch
-  int cpg;                // CTAs per batch group
+  int cpg;                // CTAs per batch group (rec_turns.cuh: per set of `turns` groups)
+  int turns;
   const bf16* W;          // [d, d], row = output feature (backward: the transposed matrix)
   const bf16* in0;        // forward pre            backward g
   const bf16* in1;        // forward g              backward dy
@@ -379,6 +380,25 @@ struct KRange {
   __device__ __forceinline__ bool owns(int kb) const { return any && col + kb * 32 >= own; }
 };
 
+// A lane's A fragments of MT tiles of W [d, d] from row `row0` on, over the warp's K range.
+template <int MT, int KB>
+__device__ __forceinline__ void load_weights(uint32_t (&w)[MT][KB][8], const bf16* W, int row0, int d,
+                                             const KRange<KB>& k) {
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+    for (int kb = 0; kb < KB; ++kb)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int row = row0 + mt * 16 + 8 * u;
+        uint4 x = make_uint4(0, 0, 0, 0);
+        if (row < d && k.owns(kb))
+          x = __ldg(reinterpret_cast<const uint4*>(W + (long)row * d + k.col + kb * 32));
+        w[mt][kb][0 + u] = x.x; w[mt][kb][2 + u] = x.y;
+        w[mt][kb][4 + u] = x.z; w[mt][kb][6 + u] = x.w;
+      }
+}
+
 }  // namespace rr
 
 template <bool BWD, int MT, int KB, int NT>
@@ -401,19 +421,7 @@ __global__ void __launch_bounds__(RR_THREADS, 1) rec_reg_kernel(const RecRegPara
   // ---- my part of W, once: rows f0 .. f0+R, this warp's KB blocks of 32 columns ----
   const rr::KRange<KB> k(d, warp, tq);
   uint32_t w[MT][KB][8];
-#pragma unroll
-  for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-    for (int kb = 0; kb < KB; ++kb)
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int row = f0 + mt * 16 + gq + 8 * u;
-        uint4 x = make_uint4(0, 0, 0, 0);
-        if (row < d && k.owns(kb))
-          x = __ldg(reinterpret_cast<const uint4*>(p.W + (long)row * d + k.col + kb * 32));
-        w[mt][kb][0 + u] = x.x; w[mt][kb][2 + u] = x.y;
-        w[mt][kb][4 + u] = x.z; w[mt][kb][6 + u] = x.w;
-      }
+  rr::load_weights(w, p.W, f0 + gq, d, k);
   // a row past the batch reads the last row's state: its products are discarded
   uint32_t x_off[NT];
 #pragma unroll

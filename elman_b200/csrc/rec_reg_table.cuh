@@ -1,7 +1,7 @@
 // Run-time (MT, KB, NT) -> instantiation of rec_reg_kernel; null outside the register budget.
 #pragma once
 
-#include "rec_reg.cuh"
+#include "rec_turns.cuh"
 
 namespace elman {
 
@@ -9,7 +9,28 @@ typedef void (*RecRegKernel)(const RecRegParams);
 RecRegKernel rec_reg_fwd_kernel(int mt, int kb, int nt);
 RecRegKernel rec_reg_bwd_kernel(int mt, int kb, int nt);
 
+// the same for rec_turns_kernel, with the most rows of W that the registers hold
+RecRegKernel rec_turns_fwd_kernel(int kb);
+RecRegKernel rec_turns_bwd_kernel(int kb);
+
 namespace rr {
+
+constexpr int turns_mt(int kb) { return kb <= RR_MAX_W / RR_MAX_MT ? RR_MAX_MT : RR_MAX_W / kb; }
+
+template <bool BWD>
+RecRegKernel pick_turns(int kb) {
+  switch (kb) {
+    case 1: return rec_turns_kernel<BWD, turns_mt(1), 1>;
+    case 2: return rec_turns_kernel<BWD, turns_mt(2), 2>;
+    case 3: return rec_turns_kernel<BWD, turns_mt(3), 3>;
+    case 4: return rec_turns_kernel<BWD, turns_mt(4), 4>;
+    case 5: return rec_turns_kernel<BWD, turns_mt(5), 5>;
+    case 6: return rec_turns_kernel<BWD, turns_mt(6), 6>;
+    case 7: return rec_turns_kernel<BWD, turns_mt(7), 7>;
+    case 8: return rec_turns_kernel<BWD, turns_mt(8), 8>;
+  }
+  return nullptr;
+}
 
 template <bool BWD, int MT, int KB, int NT>
 RecRegKernel one() {
