@@ -209,8 +209,8 @@ static bool dense_tc_ok(int dtype, int T, int B, int d, int bwd) {
   return use_tc(dtype) && rec_tc_supported(T, B, d, bwd);
 }
 
-static bool reg_ok(int dtype, int T, int B, int d) {
-  return use_tc(dtype) && rec_reg_supported(T, B, d);
+static bool reg_ok(int dtype, int T, int B, int d, int compact) {
+  return use_tc(dtype) && rec_reg_supported(T, B, d, compact);
 }
 
 // ---------------------------------------------------------------------------
@@ -246,7 +246,7 @@ static int run_rec_fwd(int dtype, int T, int B, int d, const void* W, const void
   PhaseTimer timer(0, st);
   RecFwdArgs a{T, B, d, W, pre, g, h, y, v, sync};
   a.compact = compact;
-  if (reg_ok(dtype, T, B, d)) {
+  if (reg_ok(dtype, T, B, d, compact)) {
     const int rc = rec_fwd_reg(a, st);
     if (rc != ELMAN_ERR_UNSUPPORTED) return rc;   // an unaligned operand: nothing was launched
   }
@@ -279,7 +279,7 @@ static int run_rec_bwd(int dtype, int T, int B, int d, const void* Wt, const voi
   PhaseTimer timer(1, st);
   RecBwdArgs a{T, B, d, Wt, h, v, g, dy, dv, dg, db, sync};
   a.compact = compact;
-  if (reg_ok(dtype, T, B, d)) {
+  if (reg_ok(dtype, T, B, d, compact)) {
     const int rc = rec_bwd_reg(a, st);
     if (rc != ELMAN_ERR_UNSUPPORTED) return rc;
   }
@@ -385,7 +385,7 @@ long elman_b200_tc_launch_count(void) { return g_tc_launches.load(); }
 int elman_b200_recurrence_blocks(int dtype, int flags, int T, int B, int d) {
   if (T <= 0 || B <= 0 || d <= 0) return 0;
   const int compact = (flags & ELMAN_FLAG_COMPACT) ? 1 : 0;
-  if (reg_ok(dtype, T, B, d)) return rec_reg_blocks(B, d, compact);
+  if (reg_ok(dtype, T, B, d, compact)) return rec_reg_blocks(T, B, d, compact);
   return dense_tc_ok(dtype, T, B, d, 0) && dense_tc_ok(dtype, T, B, d, 1)
              ? rec_tc_blocks(T, B, d, compact) : 0;
 }

@@ -259,12 +259,12 @@ size_t rec_tc_sync_bytes();
 int rec_fwd_tc(const RecFwdArgs& a, cudaStream_t stream);
 int rec_bwd_tc(const RecBwdArgs& a, cudaStream_t stream);
 
-// Dense recurrence, bf16, W in registers (rec_reg.cuh): up to RR_MAX_BATCH rows, d % 8 == 0,
-// d <= 2048.  Launches that may overlap others have d >= RR_MIN_CONCURRENT_D.
+// Dense recurrence, bf16, W in registers: d % 8 == 0, d <= 2048; up to RR_MAX_BATCH rows with CTAs for
+// every batch group (rec_reg.cuh), beyond that with groups that take turns (rec_turns.cuh).  Launches that may overlap others have d >= RR_MIN_CONCURRENT_D.
 constexpr int RR_MAX_BATCH = 64;
 constexpr int RR_MIN_CONCURRENT_D = 128;
-bool rec_reg_supported(int T, int B, int d);
-int rec_reg_blocks(int B, int d, int compact);
+bool rec_reg_supported(int T, int B, int d, int compact);
+int rec_reg_blocks(int T, int B, int d, int compact);
 int rec_fwd_reg(const RecFwdArgs& a, cudaStream_t stream);
 int rec_bwd_reg(const RecBwdArgs& a, cudaStream_t stream);
 // Dense recurrence, fp32, W in registers (rec_f32.cu).

@@ -75,30 +75,59 @@ RecRegPlan pick_rec_reg_plan(int B, int d) {
   return best;
 }
 
+// Sets of batch groups, each on CTAs of its own and taking turns there, on at most `ctas` CTAs.
+// (Copies of the grid over shares of the batch: option rec_replicas limits them as it does those of
+// the TMEM kernel.)
+RecRegPlan turns_plan(int B, int d, int ctas) {
+  RecRegPlan pl{};
+  pl.kb = ((d + 31) / 32 + RR_WARPS - 1) / RR_WARPS;
+  pl.ok = false;
+  if (B < 1 || d < 8 || (d & 7) != 0 || pl.kb > RR_MAX_KB) return pl;
+  pl.mt = rr::turns_mt(pl.kb);
+  pl.nt = 1;
+  pl.cpg = (d + 16 * pl.mt - 1) / (16 * pl.mt);
+  const int groups = (B + 7) / 8;
+  int sets = ctas / pl.cpg;
+  if (sets > REC_MAX_DB_ROWS) sets = REC_MAX_DB_ROWS;
+  if (options().rec_replicas > 0 && sets > options().rec_replicas) sets = (int)options().rec_replicas;
+  sets = sets < 1 ? 1 : sets > groups ? groups : sets;
+  pl.turns = (groups + sets - 1) / sets;
+  pl.groups = (groups + pl.turns - 1) / pl.turns;
+  if (pl.turns == 1) pl.turns = 0;
+  pl.ok = pl.groups * pl.cpg <= rec_reg_sms();
+  return pl;
+}
+
 // The plan for callers that overlap launches: the most rows of W per CTA, and as many of the batch
 // groups on one set of CTAs as make the launch a sixth of the device, so that six fit (the pipelined
 // model runs up to one per layer).  Measured, one optimizer step in ms with one set / with two:
 // d 1280 B 32, six layers, 20 / 40 CTAs 11.52 / 11.62; d 768 B 13, six layers, 12 / 24 CTAs 3.32 /
 // 3.23; d 256 B 32, four layers, 4 / 8 CTAs 1.64 / 1.54.  Where every group has its own CTAs this
 // is rec_reg_kernel; a plan with more CTAs than the fast one is of no use.
-RecRegPlan pick_compact_plan(int B, int d) {
-  const RecRegPlan fast = pick_rec_reg_plan(B, d);
-  if (!fast.ok) return fast;
-  RecRegPlan pl = fast;
-  pl.mt = rr::turns_mt(pl.kb);
-  pl.nt = 1;
-  pl.cpg = (d + 16 * pl.mt - 1) / (16 * pl.mt);
-  const int groups = (B + 7) / 8;
-  int sets = rec_reg_sms() / 6 / pl.cpg;
-  sets = sets < 1 ? 1 : sets > groups ? groups : sets;
-  pl.turns = (groups + sets - 1) / sets;
-  pl.groups = (groups + pl.turns - 1) / pl.turns;
-  if (pl.turns == 1) pl.turns = 0;
-  return pl.groups * pl.cpg <= fast.groups * fast.cpg ? pl : fast;
+RecRegPlan pick_compact_plan(int B, int d, const RecRegPlan& fast) {
+  const RecRegPlan pl = turns_plan(B, d, rec_reg_sms() / 6);
+  return pl.ok && pl.groups * pl.cpg <= fast.groups * fast.cpg ? pl : fast;
 }
 
-RecRegPlan plan_for(int B, int d, int compact) {
-  return compact ? pick_compact_plan(B, d) : pick_rec_reg_plan(B, d);
+// Batches with more groups than the device has room for take turns on all of it, up to where the TMEM
+// kernel, which needs about the same time for 64 rows as for 32, is ahead: 512 rows, or six turns where a
+// CTA holds 32 rows of W instead of 64 or 48 (d > 1536).  us per step forward / backward, TMEM kernel and
+// turns:
+//
+//    B    d   TMEM kernel    turns              B    d   TMEM kernel    turns
+//   128   512   4.66  4.97   1.19  1.59        256  1536   8.55  9.09   6.70  7.26
+//   256   768   5.18  5.44   2.39  2.54        512  1536  16.8  17.7   13.1  14.1
+//   128  1024   5.69  5.75   2.14  2.31         64  2048   6.18  6.37   3.75  4.02
+//   512  1024  14.9  15.4    6.59  6.92         96  2048   5.93  6.13   5.45  5.81
+//   128  1280   5.66  5.91   2.96  3.17        128  2048   6.21  5.74   7.10  7.61
+//   512  1280  10.7  10.1    9.15  9.60        256   952   350   235    3.51  3.77   (CUDA cores)
+RecRegPlan plan_for(int T, int B, int d, int compact) {
+  const RecRegPlan fast = pick_rec_reg_plan(B, d);
+  if (fast.ok) return compact ? pick_compact_plan(B, d, fast) : fast;
+  RecRegPlan pl = turns_plan(B, d, rec_reg_sms());
+  const bool slow = compact || B > 512 || (pl.kb > 6 && pl.turns > 6);
+  if (pl.ok && slow && rec_tc_supported(T, B, d, 0) && rec_tc_supported(T, B, d, 1)) pl.ok = false;
+  return pl;
 }
 
 // Options that select a plan of the TMEM kernel select that kernel.
@@ -164,17 +193,17 @@ int rec_reg_sms() {
   return sms[dev];
 }
 
-bool rec_reg_supported(int T, int B, int d) {
-  return T >= 1 && rr_enabled() && pick_rec_reg_plan(B, d).ok;
+bool rec_reg_supported(int T, int B, int d, int compact) {
+  return T >= 1 && rr_enabled() && plan_for(T, B, d, compact).ok;
 }
 
-int rec_reg_blocks(int B, int d, int compact) {
-  const RecRegPlan pl = plan_for(B, d, compact);
+int rec_reg_blocks(int T, int B, int d, int compact) {
+  const RecRegPlan pl = plan_for(T, B, d, compact);
   return pl.ok && d >= RR_MIN_CONCURRENT_D ? pl.groups * pl.cpg : 0;
 }
 
 int rec_fwd_reg(const RecFwdArgs& a, cudaStream_t stream) {
-  const RecRegPlan pl = plan_for(a.B, a.d, a.compact);
+  const RecRegPlan pl = plan_for(a.T, a.B, a.d, a.compact);
   if (!pl.ok) return ELMAN_ERR_UNSUPPORTED;
   RecRegParams p{};
   p.T = a.T; p.B = a.B; p.d = a.d;
@@ -186,7 +215,7 @@ int rec_fwd_reg(const RecFwdArgs& a, cudaStream_t stream) {
 }
 
 int rec_bwd_reg(const RecBwdArgs& a, cudaStream_t stream) {
-  const RecRegPlan pl = plan_for(a.B, a.d, a.compact);
+  const RecRegPlan pl = plan_for(a.T, a.B, a.d, a.compact);
   if (!pl.ok) return ELMAN_ERR_UNSUPPORTED;
   RecRegParams p{};
   p.T = a.T; p.B = a.B; p.d = a.d;

@@ -170,9 +170,8 @@ int elman_e1_backward(int dtype, int T, int B, int d,
 /*
  * elman_e1_forward with launch flags (an extension; elman_e1_forward is flags 0).
  *   ELMAN_FLAG_COMPACT  run the recurrence with the plan that keeps the fewest thread
- *                       blocks resident (a smaller split of the reduction dimension, the
- *                       weight tile in tensor memory where shared memory cannot hold it)
- *                       instead of the plan with the shortest step.  For callers that
+ *                       blocks resident (batch groups that take turns on one set of blocks, or
+ *                       a smaller split of the reduction dimension) instead of the plan with the shortest step.  For callers that
  *                       overlap several recurrence launches on different streams: a step
  *                       gets somewhat slower, the launch leaves more of the GPU to others.
  * Results differ from flags 0 only by the summation order of the split reduction.

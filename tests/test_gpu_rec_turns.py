@@ -37,6 +37,27 @@ def test_ragged_shapes_match_oracle(T, B, d):
     assert_close(errors(got, oracle_e1(ref)), TOL[torch.bfloat16], f"T{T} B{B} d{d}")
 
 
+@pytest.mark.parametrize("T,B,d", [(4, 65, 64), (3, 130, 520), (3, 100, 952), (2, 250, 1280), (2, 90, 2048),
+                                   (3, 64, 1792)])
+def test_large_batches_match_oracle(T, B, d):
+    """Without the flag: more groups than the device has CTAs for; E1, E1 without a backward pass,
+    and the state as its own gate (E33)."""
+    inp = orc.make_e1_inputs(T, B, d, seed=d - B)
+    got, ref = run_compact(inp, 0)
+    assert _lib.device_status()[0] == 0
+    assert_close(errors(got, oracle_e1(ref)), TOL[torch.bfloat16], f"T{T} B{B} d{d}")
+    dev, _ = round_inputs(inp, torch.bfloat16)
+    h, out, _ = H.mamba_gated_elman_forward(False, dev["x"], dev["z"], dev["h0"], dev["W_x"], dev["W_h"],
+                                            dev["b"])
+    assert torch.equal(h, got["h"]) and torch.equal(out, got["output"])
+    h, out, v = H.e33_self_gate_forward(True, dev["x"], dev["h0"], dev["W_x"], dev["W_h"], dev["b"])
+    dx, dWx, dWh, db = H.e33_self_gate_backward(dev["W_x"], dev["W_h"], dev["x"], h, v, dev["d_output"])
+    f = orc.e33_forward(ref["x"], ref["h0"], ref["W_x"], ref["W_h"], ref["b"])
+    g = orc.e33_backward(ref["W_x"], ref["W_h"], ref["x"], f["h"], f["v"], ref["d_output"])
+    assert_close(errors(dict(h=h, output=out, v=v, dx=dx, dW_x=dWx, dW_h=dWh, db=db), {**f, **g}),
+                 TOL[torch.bfloat16], "self gate")
+
+
 def test_long_chain_agrees_with_one_group_per_set():
     """300 steps, many rounds of the ring and the buffers, against the kernel without turns."""
     inp = orc.make_e1_inputs(300, 29, 1280, seed=1)
