@@ -17,12 +17,13 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import _lib, _spectral, fused_ops
-from .mamba_gated_elman import MambaGatedElman
+from .mamba_gated_elman import MambaGatedElman, MambaGatedElmanCell
 from .pure_lowrank_elman import PureLowRankElman
 from .siblings import E32NoPresilu, E33SelfGate, E57LearnedRadius, LowRankElman
 from .stock_elman import StockElman
 
 _NO_SWITCH = contextlib.nullcontext()
+_PLAIN_TENSORS = {torch.Tensor, nn.Parameter}
 
 _LEVELS = {0: StockElman, 1: MambaGatedElman, 4: LowRankElman, 5: PureLowRankElman,
            32: E32NoPresilu, 33: E33SelfGate, 57: E57LearnedRadius}
@@ -162,30 +163,16 @@ class LadderLM(nn.Module):
         every call, by the shortest way (dictionaries instead of nn.Module attribute access); what
         follows from them alone is checked again only when one of their addresses or types is not
         the one it was."""
-        mods = self._modules
-        emb = mods["embedding"]._parameters["weight"]
-        dtype, d = emb.dtype, self.dim
-        if dtype is not torch.bfloat16 or not emb.is_cuda or not self.fused_ops \
-                or inp.dtype is not torch.int64 or not inp.is_cuda:
+        operands = self._token_operands()
+        if operands is None:
             return None
-        params, addresses = [emb], []
-        vectors, eps = [], [mods["norm"].eps]
-        for layer, ln in zip(mods["layers"]._modules.values(), mods["layer_norms"]._modules.values()):
-            lm = layer._modules
-            cell = lm.get("cell")
-            if type(layer) is not MambaGatedElman or layer.use_conv or not layer.fused \
-                    or layer.d_inner != d or (self.training and type(lm["dropout"]) is nn.Dropout):
-                return None
-            cp = cell._parameters
-            W_h = cp["W_h"]
-            params += (ln._parameters["weight"], lm["in_proj"]._parameters["weight"], cp["W_x"], W_h,
-                       cp["b"], lm["out_proj"]._parameters["weight"])
-            eps.append(ln.eps)
-            vectors.append(_spectral.library_vector(cell, W_h)
-                           if cell.w_h_mode == "spectral_norm" and W_h.is_cuda else None)
-        params += (mods["norm"]._parameters["weight"], mods["lm_head"]._parameters["weight"])
-        if not _spectral.FUSED:
+        params, eps, cells = operands
+        dtype, d = params[0].dtype, self.dim
+        if dtype is not torch.bfloat16 or not params[0].is_cuda \
+                or inp.dtype is not torch.int64 or not inp.is_cuda or not _spectral.FUSED:
             return None
+        vectors = [_spectral.library_vector(cell, W_h) if cell.w_h_mode == "spectral_norm" and W_h.is_cuda
+                   else None for cell, W_h in zip(cells, params[4::6])]
         addresses = [(p.data_ptr(), p.dtype) for p in params] + eps
         plan = self.__dict__.get("_token_plan")
         if plan is None or plan[0] != addresses:
@@ -226,6 +213,38 @@ class LadderLM(nn.Module):
             return None
         _lib.check(rc, "elman_e1_lm_token")
         return logits, list(hiddens.unbind(0))
+
+    def _token_operands(self):
+        """What the generation kernel reads: ([embedding, then per layer norm, in_proj, W_x, W_h, b,
+        out_proj, then the final norm, head], [epsilon of every norm], [cell of every layer]) — or None
+        for a model with anything else in one of these places.  A parametrised or pruned weight is no
+        entry of `_parameters`: the module computes it."""
+        mods = self._modules
+        emb, norm, head = mods.get("embedding"), mods.get("norm"), mods.get("lm_head")
+        if not self.fused_ops or type(emb) is not nn.Embedding or type(norm) is not nn.RMSNorm \
+                or type(head) is not nn.Linear:
+            return None
+        d = self.dim
+        params = [emb._parameters.get("weight")]
+        eps, cells = [norm.eps], []
+        for layer, ln in zip(mods["layers"]._modules.values(), mods["layer_norms"]._modules.values()):
+            if type(layer) is not MambaGatedElman or layer.use_conv or not layer.fused \
+                    or layer.d_inner != d or (self.training and type(layer._modules["dropout"]) is nn.Dropout):
+                return None
+            lm = layer._modules
+            cell, w_in, w_out = lm.get("cell"), lm.get("in_proj"), lm.get("out_proj")
+            if type(cell) is not MambaGatedElmanCell or type(w_in) is not nn.Linear \
+                    or type(w_out) is not nn.Linear or type(ln) is not nn.RMSNorm:
+                return None
+            cp = cell._parameters
+            params += (ln._parameters.get("weight"), w_in._parameters.get("weight"), cp.get("W_x"),
+                       cp.get("W_h"), cp.get("b"), w_out._parameters.get("weight"))
+            eps.append(ln.eps)
+            cells.append(cell)
+        params += (norm._parameters.get("weight"), head._parameters.get("weight"))
+        if not _PLAIN_TENSORS.issuperset(map(type, params)):     # None, or a tensor with a mind of its own
+            return None
+        return params, eps, cells
 
     def _token_plan_for(self, params):
         """(pointer table without the per-call entries, device, epsilon) of the generation kernel, or

@@ -1,0 +1,61 @@
+"""What LadderLM hands to the generation kernel (csrc/lm_token.cu): models that ask for anything the
+kernel does not compute go layer by layer, with the results and side effects that path has."""
+import pytest
+import torch
+import torch.nn as nn
+
+from _gpu_cases import TOL, option
+from elman_b200 import _lib
+from elman_b200.ladder_lm import LadderLM
+from oracle import elman_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+TOKENS = [[3], [250], [77]]
+
+
+def _model(d=64, depth=2, seed=5, **kw):
+    torch.manual_seed(seed)
+    return LadderLM(vocab_size=256, dim=d, depth=depth, level=1, **{"r_h_mode": "none", **kw}).cuda().bfloat16().eval()
+
+
+def _tokens():
+    return torch.tensor(TOKENS).cuda()
+
+
+@torch.no_grad()
+def _one_token(model, tokens=None):
+    """(logits, launches of the library)"""
+    before = _lib.launch_count()
+    logits = model(_tokens() if tokens is None else tokens)
+    torch.cuda.synchronize()
+    return logits, _lib.launch_count() - before
+
+
+def _layer_by_layer(model, tokens=None):
+    with option("rec_reg", 1):     # no register kernels: the generation kernel steps aside
+        return _one_token(model, tokens)[0]
+
+
+def _close(a, b):
+    return a.shape == b.shape and orc.rel_err(a.float().cpu(), b.float().cpu()) < TOL[torch.bfloat16]
+
+
+def test_plain_model_takes_the_kernel():
+    model = _model()
+    logits, launches = _one_token(model)
+    assert launches <= 2 and _close(logits, _layer_by_layer(model))
+
+
+@pytest.mark.parametrize("where", ["embedding", "norm", "W_h", "in_proj"])
+def test_parametrised_weights_go_layer_by_layer(where):
+    from torch.nn.utils import parametrizations, prune
+    model = _model()
+    if where == "W_h":
+        prune.random_unstructured(model.layers[1].cell, "W_h", amount=0.5)
+    elif where == "norm":
+        prune.random_unstructured(model.norm, "weight", amount=0.5)
+    else:
+        parametrizations.weight_norm(model.embedding if where == "embedding" else model.layers[0].in_proj)
+    logits, launches = _one_token(model)
+    assert launches > 2 and _close(logits, _layer_by_layer(model))

@@ -1,0 +1,43 @@
+"""Which models LadderLM hands to the generation kernel, on the CPU: what it reads out of the modules
+(`_token_operands`), and that everything else reaches the layers."""
+import pytest
+import torch
+
+from elman_b200.ladder_lm import LadderLM
+
+
+def _model(level=1, **kw):
+    return LadderLM(vocab_size=256, dim=32, depth=2, level=level, **kw).bfloat16().eval()
+
+
+def _parametrise(model, where):
+    from torch.nn.utils import parametrizations, prune
+    if where == "W_h":
+        prune.random_unstructured(model.layers[1].cell, "W_h", amount=0.5)
+    elif where == "norm":
+        prune.random_unstructured(model.norm, "weight", amount=0.5)
+    else:
+        parametrizations.weight_norm(model.get_submodule(where))
+
+
+def test_plain_model():
+    model = _model()
+    params, eps, cells = model._token_operands()
+    assert [p.shape for p in params] == (
+        [(256, 32)] + 2 * [(32,), (64, 32), (32, 32), (32, 32), (32,), (32, 32)] + [(32,), (256, 32)])
+    assert cells == [layer.cell for layer in model.layers]
+
+
+@pytest.mark.parametrize("where", ["embedding", "norm", "W_h", "layers.0.in_proj", "lm_head"])
+def test_parametrised_weights(where):
+    model = _model()
+    _parametrise(model, where)
+    assert model._token_operands() is None
+
+
+@pytest.mark.parametrize("level", [0, 1])
+def test_one_token_on_the_cpu_is_refused_by_the_layer(level):
+    model = _model(level)
+    _parametrise(model, "embedding")
+    with torch.no_grad(), pytest.raises(RuntimeError, match="CUDA"):
+        model(torch.tensor([[3]]))
