@@ -229,9 +229,12 @@ class LadderLM(nn.Module):
         eps, cells = [norm.eps], []
         for layer, ln in zip(mods["layers"]._modules.values(), mods["layer_norms"]._modules.values()):
             if type(layer) is not MambaGatedElman or layer.use_conv or not layer.fused \
-                    or layer.d_inner != d or (self.training and type(layer._modules["dropout"]) is nn.Dropout):
+                    or layer.d_inner != d:
                 return None
             lm = layer._modules
+            drop = lm.get("dropout")      # its own switch decides, not the model's
+            if type(drop) is not nn.Identity and (type(drop) is not nn.Dropout or drop.training):
+                return None
             cell, w_in, w_out = lm.get("cell"), lm.get("in_proj"), lm.get("out_proj")
             if type(cell) is not MambaGatedElmanCell or type(w_in) is not nn.Linear \
                     or type(w_out) is not nn.Linear or type(ln) is not nn.RMSNorm:

@@ -59,3 +59,24 @@ def test_parametrised_weights_go_layer_by_layer(where):
         parametrizations.weight_norm(model.embedding if where == "embedding" else model.layers[0].in_proj)
     logits, launches = _one_token(model)
     assert launches > 2 and _close(logits, _layer_by_layer(model))
+
+
+def test_dropout_that_is_training_drops():
+    model = _model(dropout=0.5)
+    model.eval()
+    assert torch.equal(_one_token(model)[0], _one_token(model)[0])
+    for layer in model.layers:
+        layer.dropout.train()          # Monte Carlo dropout
+    assert not torch.equal(_one_token(model)[0], _one_token(model)[0])
+
+
+def test_replaced_modules_are_called():
+    class Halve(nn.Module):
+        def forward(self, x):
+            return 0.5 * x
+
+    model = _model()
+    plain, _ = _one_token(model)
+    model.layers[0].dropout = Halve()
+    logits, _ = _one_token(model)
+    assert not torch.equal(logits, plain) and _close(logits, _layer_by_layer(model))

@@ -41,3 +41,20 @@ def test_one_token_on_the_cpu_is_refused_by_the_layer(level):
     _parametrise(model, "embedding")
     with torch.no_grad(), pytest.raises(RuntimeError, match="CUDA"):
         model(torch.tensor([[3]]))
+
+
+def test_dropout_that_is_training():
+    model = _model(dropout=0.5)
+    assert model._token_operands() is not None
+    model.layers[1].dropout.train()             # the model itself still in eval()
+    assert model._token_operands() is None
+    model.train().layers[1].dropout.eval()
+    assert model._token_operands() is None       # layer 0
+    model.layers[0].dropout.eval()
+    assert model._token_operands() is not None
+
+
+def test_replaced_dropout():
+    model = _model()
+    model.layers[0].dropout = torch.nn.Tanh()
+    assert model._token_operands() is None
