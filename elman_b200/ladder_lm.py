@@ -24,6 +24,13 @@ from .stock_elman import StockElman
 
 _NO_SWITCH = contextlib.nullcontext()
 _PLAIN_TENSORS = {torch.Tensor, nn.Parameter}
+_module = nn.modules.module
+
+
+def _runs_only(module, cls):
+    """Calling `module` is cls.forward and nothing else: no subclass, no hook, no forward of its own."""
+    return (type(module) is cls and not module._forward_hooks and not module._forward_pre_hooks
+            and "forward" not in module.__dict__)
 
 _LEVELS = {0: StockElman, 1: MambaGatedElman, 4: LowRankElman, 5: PureLowRankElman,
            32: E32NoPresilu, 33: E33SelfGate, 57: E57LearnedRadius}
@@ -221,22 +228,25 @@ class LadderLM(nn.Module):
         entry of `_parameters`: the module computes it."""
         mods = self._modules
         emb, norm, head = mods.get("embedding"), mods.get("norm"), mods.get("lm_head")
-        if not self.fused_ops or type(emb) is not nn.Embedding or type(norm) is not nn.RMSNorm \
-                or type(head) is not nn.Linear:
+        # the layers' path calls the embedding, the layers, their cells and dropout modules; of the
+        # others it reads the weights
+        if type(self) is not LadderLM or not self.fused_ops or _module._global_forward_hooks \
+                or _module._global_forward_pre_hooks or not _runs_only(emb, nn.Embedding) \
+                or emb.max_norm is not None or type(norm) is not nn.RMSNorm or type(head) is not nn.Linear:
             return None
         d = self.dim
         params = [emb._parameters.get("weight")]
         eps, cells = [norm.eps], []
         for layer, ln in zip(mods["layers"]._modules.values(), mods["layer_norms"]._modules.values()):
-            if type(layer) is not MambaGatedElman or layer.use_conv or not layer.fused \
+            if not _runs_only(layer, MambaGatedElman) or layer.use_conv or not layer.fused \
                     or layer.d_inner != d:
                 return None
             lm = layer._modules
             drop = lm.get("dropout")      # its own switch decides, not the model's
-            if type(drop) is not nn.Identity and (type(drop) is not nn.Dropout or drop.training):
+            if not _runs_only(drop, nn.Identity) and (not _runs_only(drop, nn.Dropout) or drop.training):
                 return None
             cell, w_in, w_out = lm.get("cell"), lm.get("in_proj"), lm.get("out_proj")
-            if type(cell) is not MambaGatedElmanCell or type(w_in) is not nn.Linear \
+            if not _runs_only(cell, MambaGatedElmanCell) or type(w_in) is not nn.Linear \
                     or type(w_out) is not nn.Linear or type(ln) is not nn.RMSNorm:
                 return None
             cp = cell._parameters

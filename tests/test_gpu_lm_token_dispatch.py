@@ -80,3 +80,22 @@ def test_replaced_modules_are_called():
     model.layers[0].dropout = Halve()
     logits, _ = _one_token(model)
     assert not torch.equal(logits, plain) and _close(logits, _layer_by_layer(model))
+
+
+@pytest.mark.parametrize("kind", ["forward", "pre", "global"])
+@pytest.mark.parametrize("where", ["embedding", "layers.1", "layers.0.cell", "layers.1.dropout"])
+def test_hooks_fire(where, kind):
+    model = _model(dropout=0.1)
+    module, calls = model.get_submodule(where), []
+    if kind == "forward":
+        handle = module.register_forward_hook(lambda m, *a: calls.append(m))
+    elif kind == "pre":
+        handle = module.register_forward_pre_hook(lambda m, *a: calls.append(m))
+    else:
+        handle = nn.modules.module.register_module_forward_hook(
+            lambda m, *a: calls.append(m) if m is module else None)
+    try:
+        _one_token(model)
+    finally:
+        handle.remove()
+    assert calls == [module]

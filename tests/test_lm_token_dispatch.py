@@ -58,3 +58,40 @@ def test_replaced_dropout():
     model = _model()
     model.layers[0].dropout = torch.nn.Tanh()
     assert model._token_operands() is None
+
+
+@pytest.mark.parametrize("kind", ["forward", "pre", "global", "global pre"])
+@pytest.mark.parametrize("where", ["embedding", "layers.1", "layers.0.cell", "layers.1.dropout"])
+def test_hooks(where, kind):
+    model = _model(dropout=0.1)
+    module, hooks = model.get_submodule(where), torch.nn.modules.module
+    register = {"forward": module.register_forward_hook, "pre": module.register_forward_pre_hook,
+                "global": hooks.register_module_forward_hook,
+                "global pre": hooks.register_module_forward_pre_hook}[kind]
+    handle = register(lambda *a: None)
+    try:
+        assert model._token_operands() is None
+    finally:
+        handle.remove()
+    assert model._token_operands() is not None
+
+
+@pytest.mark.parametrize("where", ["embedding", "layers.1", "layers.0.cell", "layers.1.dropout"])
+def test_other_classes_and_forwards_of_their_own(where):
+    model = _model()
+    module = model.get_submodule(where)
+    module.forward = module.forward
+    assert model._token_operands() is None
+    del module.forward
+    assert model._token_operands() is not None
+    module.__class__ = type("Mine", (type(module),), {})
+    assert model._token_operands() is None
+
+
+def test_subclass_and_renormalised_embedding():
+    model = _model()
+    model.embedding.max_norm = 1.0
+    assert model._token_operands() is None
+    model = _model()
+    model.__class__ = type("Mine", (LadderLM,), {})     # may override _add_norm, _head
+    assert model._token_operands() is None
