@@ -11,6 +11,7 @@ ignored.
 """
 import contextlib
 import ctypes
+import operator
 
 import torch
 import torch.nn as nn
@@ -24,6 +25,8 @@ from .stock_elman import StockElman
 
 _NO_SWITCH = contextlib.nullcontext()
 _PLAIN_TENSORS = {torch.Tensor, nn.Parameter}
+_DTYPE = operator.attrgetter("dtype")
+_DATA_PTR = torch.Tensor.data_ptr
 _module = nn.modules.module
 
 
@@ -166,54 +169,46 @@ class LadderLM(nn.Module):
         library's generation kernel: (logits [B,1,V], [final state of every layer]) — or None
         when the model or the tensors are not what that kernel takes.
 
-        Issuing the step must not take longer than the step.  The parameters are looked up anew on
-        every call, by the shortest way (dictionaries instead of nn.Module attribute access); what
-        follows from them alone is checked again only when one of their addresses or types is not
-        the one it was."""
+        Issuing the step must not take longer than the step, so everything is looked up and checked by
+        the shortest way (dictionaries instead of nn.Module attribute access, one pass over all
+        parameters per question) — but on every call, and nothing is kept for the next one."""
         operands = self._token_operands()
         if operands is None:
             return None
         params, eps, cells = operands
-        dtype, d = params[0].dtype, self.dim
-        if dtype is not torch.bfloat16 or not params[0].is_cuda \
-                or inp.dtype is not torch.int64 or not inp.is_cuda or not _spectral.FUSED:
-            return None
-        vectors = [_spectral.library_vector(cell, W_h) if cell.w_h_mode == "spectral_norm" and W_h.is_cuda
-                   else None for cell, W_h in zip(cells, params[4::6])]
-        addresses = [(p.data_ptr(), p.dtype) for p in params] + eps
-        plan = self.__dict__.get("_token_plan")
-        if plan is None or plan[0] != addresses:
-            plan = self.__dict__["_token_plan"] = (addresses, *self._token_plan_for(params))
-        _, table0, device, eps = plan
-        if table0 is None or inp.device != device:
+        device, d = params[0].device, self.dim
+        if device.type != "cuda" or inp.dtype is not torch.int64 or inp.device != device \
+                or not _spectral.FUSED:
             return None
         B, depth, V = inp.size(0), self.depth, self.vocab_size
         lib = _lib.load()
         if not lib.elman_e1_lm_token_supported(_lib.ELMAN_BF16, depth, B, d, V):
             return None
-        table = type(table0).from_buffer_copy(table0)
-        hiddens = torch.empty(depth, B, d, dtype=dtype, device=device)
+        addresses = list(map(_DATA_PTR, params))
+        hiddens = torch.empty(depth, B, d, dtype=torch.bfloat16, device=device)
         h_out, h_bytes, shape = hiddens.data_ptr(), B * d * 2, (B, d)
-        keep = []
-        for i, (h, u) in enumerate(zip(prev_hiddens, vectors)):
-            at = 9 * i + 6
-            if u is not None:
-                table[at] = u.data_ptr()
+        keep, table = [], []
+        for i, (h, cell) in enumerate(zip(prev_hiddens, cells)):
+            table += addresses[1 + 6 * i:7 + 6 * i]
+            table.append(_spectral.library_vector(cell, params[4 + 6 * i]).data_ptr()
+                         if cell.w_h_mode == "spectral_norm" else None)
             if h is not None:
-                if h.dtype is not dtype or h.device != device or h.shape != shape:
+                if h.dtype is not torch.bfloat16 or h.device != device or h.shape != shape:
                     return None
                 if not h.is_contiguous():
                     h = h.contiguous()
                     keep.append(h)
-                table[at + 1] = h.data_ptr()
-            table[at + 2] = h_out + i * h_bytes
+                h = h.data_ptr()
+            table.append(h)
+            table.append(h_out + i * h_bytes)
         tokens = inp.contiguous()
-        logits = torch.empty(B, 1, V, dtype=dtype, device=device)
+        logits = torch.empty(B, 1, V, dtype=torch.bfloat16, device=device)
         with torch.cuda.device(device) if torch.cuda.current_device() != device.index else _NO_SWITCH:
             ws = torch.empty(lib.elman_e1_lm_token_workspace(depth, B, d), dtype=torch.uint8, device=device)
             rc = lib.elman_e1_lm_token(
-                _lib.ELMAN_BF16, depth, B, d, V, tokens.data_ptr(), addresses[0][0], table,
-                params[-2].data_ptr(), params[-1].data_ptr(), eps, _spectral.TARGET_RADIUS, _spectral.EPS,
+                _lib.ELMAN_BF16, depth, B, d, V, tokens.data_ptr(), addresses[0],
+                (ctypes.c_void_p * len(table))(*table), addresses[-2], addresses[-1],
+                eps, _spectral.TARGET_RADIUS, _spectral.EPS,
                 logits.data_ptr(), ws.data_ptr(), ws.numel(),
                 torch.cuda.current_stream(device).cuda_stream)
         if rc == _lib.ELMAN_ERR_UNSUPPORTED:     # an operand off its 16-byte boundary
@@ -223,7 +218,7 @@ class LadderLM(nn.Module):
 
     def _token_operands(self):
         """What the generation kernel reads: ([embedding, then per layer norm, in_proj, W_x, W_h, b,
-        out_proj, then the final norm, head], [epsilon of every norm], [cell of every layer]) — or None
+        out_proj, then the final norm, head], the norms' epsilon, [cell of every layer]) — or None
         for a model with anything else in one of these places.  A parametrised or pruned weight is no
         entry of `_parameters`: the module computes it."""
         mods = self._modules
@@ -236,7 +231,7 @@ class LadderLM(nn.Module):
             return None
         d = self.dim
         params = [emb._parameters.get("weight")]
-        eps, cells = [norm.eps], []
+        eps, cells = norm.eps, []
         for layer, ln in zip(mods["layers"]._modules.values(), mods["layer_norms"]._modules.values()):
             if not _runs_only(layer, MambaGatedElman) or layer.use_conv or not layer.fused \
                     or layer.d_inner != d:
@@ -247,33 +242,19 @@ class LadderLM(nn.Module):
                 return None
             cell, w_in, w_out = lm.get("cell"), lm.get("in_proj"), lm.get("out_proj")
             if not _runs_only(cell, MambaGatedElmanCell) or type(w_in) is not nn.Linear \
-                    or type(w_out) is not nn.Linear or type(ln) is not nn.RMSNorm:
+                    or type(w_out) is not nn.Linear or type(ln) is not nn.RMSNorm or ln.eps != eps:
                 return None
             cp = cell._parameters
             params += (ln._parameters.get("weight"), w_in._parameters.get("weight"), cp.get("W_x"),
                        cp.get("W_h"), cp.get("b"), w_out._parameters.get("weight"))
-            eps.append(ln.eps)
             cells.append(cell)
         params += (norm._parameters.get("weight"), head._parameters.get("weight"))
-        if not _PLAIN_TENSORS.issuperset(map(type, params)):     # None, or a tensor with a mind of its own
+        if not _PLAIN_TENSORS.issuperset(map(type, params)) \
+                or set(map(_DTYPE, params)) != {torch.bfloat16} \
+                or len(set(map(torch.Tensor.get_device, params))) != 1 \
+                or not all(map(torch.Tensor.is_contiguous, params)):
             return None
-        return params, eps, cells
-
-    def _token_plan_for(self, params):
-        """(pointer table without the per-call entries, device, epsilon) of the generation kernel, or
-        (None, None, None) when it does not take these parameters."""
-        no = (None, None, None)
-        device = params[0].device
-        if any(p.dtype != torch.bfloat16 or p.device != device or not p.is_contiguous() for p in params):
-            return no
-        norms = list(self.layer_norms) + [self.norm]
-        if any(getattr(n, "eps", None) != norms[0].eps for n in norms):
-            return no
-        table = (ctypes.c_void_p * (9 * self.depth))()
-        for i in range(self.depth):
-            for j in range(6):
-                table[9 * i + j] = params[1 + 6 * i + j].data_ptr()
-        return table, device, fused_ops.rmsnorm_eps(self.norm, torch.bfloat16)
+        return params, fused_ops.rmsnorm_eps(norm, torch.bfloat16), cells
 
     def _add_norm(self, norm, h, residual, last=False, group=None):
         """residual = h + residual (fp32 stream); h = norm(residual in the layer's dtype).

@@ -1,5 +1,8 @@
 """What LadderLM hands to the generation kernel (csrc/lm_token.cu): models that ask for anything the
 kernel does not compute go layer by layer, with the results and side effects that path has."""
+import copy
+import io
+
 import pytest
 import torch
 import torch.nn as nn
@@ -99,3 +102,24 @@ def test_hooks_fire(where, kind):
     finally:
         handle.remove()
     assert calls == [module]
+
+
+def test_transposed_weight_is_read_as_the_tensor_says():
+    model = _model()
+    _one_token(model)
+    W = model.layers[0].cell.W_x
+    W.data = W.data.t()               # the same address
+    logits, _ = _one_token(model)
+    assert _close(logits, _layer_by_layer(model))
+    model.layers[0].cell.W_x = nn.Parameter(W.detach().contiguous())
+    assert _close(logits, _one_token(model)[0])
+
+
+def test_model_is_copied_and_saved_after_a_token():
+    model = _model()
+    want, _ = _one_token(model)
+    assert torch.equal(_one_token(copy.deepcopy(model))[0], want)
+    buffer = io.BytesIO()
+    torch.save(model, buffer)
+    buffer.seek(0)
+    assert torch.equal(_one_token(torch.load(buffer, weights_only=False))[0], want)

@@ -23,6 +23,7 @@ def _parametrise(model, where):
 def test_plain_model():
     model = _model()
     params, eps, cells = model._token_operands()
+    assert eps == torch.finfo(torch.float32).eps
     assert [p.shape for p in params] == (
         [(256, 32)] + 2 * [(32,), (64, 32), (32, 32), (32, 32), (32,), (32, 32)] + [(32,), (256, 32)])
     assert cells == [layer.cell for layer in model.layers]
@@ -94,4 +95,18 @@ def test_subclass_and_renormalised_embedding():
     assert model._token_operands() is None
     model = _model()
     model.__class__ = type("Mine", (LadderLM,), {})     # may override _add_norm, _head
+    assert model._token_operands() is None
+
+
+def test_tensors_in_another_form():
+    model = _model()
+    W = model.layers[0].cell.W_x
+    W.data = W.data.t()                                   # same storage, same address
+    assert model._token_operands() is None
+    W.data = W.data.contiguous()
+    assert model._token_operands() is not None
+    model.layers[1].cell.b.data = model.layers[1].cell.b.data.float()
+    assert model._token_operands() is None
+    model = _model()
+    model.layer_norms[1].eps = 1e-3
     assert model._token_operands() is None
