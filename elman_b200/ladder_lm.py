@@ -176,11 +176,11 @@ class LadderLM(nn.Module):
         if operands is None:
             return None
         params, eps, cells = operands
-        device, d = params[0].device, self.dim
+        device, depth, (V, d) = params[0].device, len(cells), params[0].shape
         if device.type != "cuda" or inp.dtype is not torch.int64 or inp.device != device \
-                or not _spectral.FUSED:
+                or len(prev_hiddens) != depth or not _spectral.FUSED or _spectral.POWER_ITERS != 3:
             return None
-        B, depth, V = inp.size(0), self.depth, self.vocab_size
+        B = inp.size(0)
         lib = _lib.load()
         if not lib.elman_e1_lm_token_supported(_lib.ELMAN_BF16, depth, B, d, V):
             return None
@@ -229,12 +229,13 @@ class LadderLM(nn.Module):
                 or _module._global_forward_pre_hooks or not _runs_only(emb, nn.Embedding) \
                 or emb.max_norm is not None or type(norm) is not nn.RMSNorm or type(head) is not nn.Linear:
             return None
-        d = self.dim
         params = [emb._parameters.get("weight")]
         eps, cells = norm.eps, []
-        for layer, ln in zip(mods["layers"]._modules.values(), mods["layer_norms"]._modules.values()):
-            if not _runs_only(layer, MambaGatedElman) or layer.use_conv or not layer.fused \
-                    or layer.d_inner != d:
+        layers, norms = mods["layers"]._modules, mods["layer_norms"]._modules
+        if len(layers) != len(norms):
+            return None
+        for layer, ln in zip(layers.values(), norms.values()):
+            if not _runs_only(layer, MambaGatedElman) or layer.use_conv or not layer.fused:
                 return None
             lm = layer._modules
             drop = lm.get("dropout")      # its own switch decides, not the model's
@@ -253,6 +254,13 @@ class LadderLM(nn.Module):
                 or set(map(_DTYPE, params)) != {torch.bfloat16} \
                 or len(set(map(torch.Tensor.get_device, params))) != 1 \
                 or not all(map(torch.Tensor.is_contiguous, params)):
+            return None
+        # one width throughout; the vocabulary is what the tables hold
+        table, d = params[0].shape, params[-2].numel()
+        row, square = torch.Size((d,)), torch.Size((d, d))
+        want = [torch.Size((table[0], d))]
+        want += [row, torch.Size((2 * d, d)), square, square, row, square] * len(cells) + [row, want[0]]
+        if list(map(torch.Tensor.size, params)) != want:
             return None
         return params, fused_ops.rmsnorm_eps(norm, torch.bfloat16), cells
 

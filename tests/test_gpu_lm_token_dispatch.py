@@ -115,6 +115,28 @@ def test_transposed_weight_is_read_as_the_tensor_says():
     assert _close(logits, _one_token(model)[0])
 
 
+@pytest.mark.parametrize("rows", [264, 100])
+def test_vocabulary_is_that_of_the_tables(rows):
+    """Tables grown after construction (ids up to 263 are legal then), or cut."""
+    model = _model()
+    torch.manual_seed(1)
+    model.embedding = nn.Embedding(rows, 64, device="cuda", dtype=torch.bfloat16)
+    model.lm_head = nn.Linear(64, rows, bias=False, device="cuda", dtype=torch.bfloat16)
+    tokens = torch.tensor([[3], [rows - 1]]).cuda()
+    logits, _ = _one_token(model, tokens)
+    assert logits.shape == (2, 1, rows)
+    assert _lib.device_status()[0] == 0
+    assert _close(logits, _layer_by_layer(model, tokens))
+    assert _one_token(model, tokens)[1] <= 2
+
+
+def test_tables_of_different_sizes_go_layer_by_layer():
+    model = _model()
+    model.lm_head = nn.Linear(64, 8, bias=False, device="cuda", dtype=torch.bfloat16)
+    logits, launches = _one_token(model)
+    assert launches > 2 and logits.shape == (3, 1, 8)
+
+
 def test_model_is_copied_and_saved_after_a_token():
     model = _model()
     want, _ = _one_token(model)

@@ -110,3 +110,31 @@ def test_tensors_in_another_form():
     model = _model()
     model.layer_norms[1].eps = 1e-3
     assert model._token_operands() is None
+
+
+def test_tables_of_another_size():
+    nn, model = torch.nn, _model()
+    model.lm_head = nn.Linear(32, 8, bias=False, dtype=torch.bfloat16)
+    assert model._token_operands() is None
+    model.embedding = nn.Embedding(8, 32, dtype=torch.bfloat16)
+    assert model._token_operands()[0][0].shape == (8, 32)      # vocab_size is not asked
+    model.embedding = nn.Embedding(8, 40, dtype=torch.bfloat16)
+    assert model._token_operands() is None
+
+
+@pytest.mark.parametrize("name,shape", [("layers.0.cell.W_x", (32, 40)), ("layers.1.cell.b", (64,)),
+                                        ("layers.0.in_proj.weight", (32, 32)), ("layer_norms.1.weight", (8,)),
+                                        ("norm.weight", (1, 32)), ("layers.1.out_proj.weight", (32, 16))])
+def test_weights_of_another_shape(name, shape):
+    model = _model()
+    model.get_parameter(name).data = torch.zeros(shape, dtype=torch.bfloat16)
+    assert model._token_operands() is None
+
+
+def test_fewer_layers_than_it_was_built_with():
+    model = _model()
+    model.layers = model.layers[:1]
+    assert model._token_operands() is None                      # two norms, one layer
+    model.layer_norms = model.layer_norms[:1]
+    assert len(model._token_operands()[2]) == 1
+    assert _model(expansion=1.5)._token_operands() is None
