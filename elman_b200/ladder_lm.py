@@ -225,8 +225,8 @@ class LadderLM(nn.Module):
         emb, norm, head = mods.get("embedding"), mods.get("norm"), mods.get("lm_head")
         # the layers' path calls the embedding, the layers, their cells and dropout modules; of the
         # others it reads the weights
-        if type(self) is not LadderLM or not self.fused_ops or _module._global_forward_hooks \
-                or _module._global_forward_pre_hooks or not _runs_only(emb, nn.Embedding) \
+        if type(self) is not LadderLM or not self.fused_ops or not self.residual_in_fp32 \
+                or _module._global_forward_hooks or _module._global_forward_pre_hooks or not _runs_only(emb, nn.Embedding) \
                 or emb.max_norm is not None or type(norm) is not nn.RMSNorm or type(head) is not nn.Linear:
             return None
         params = [emb._parameters.get("weight")]

@@ -104,6 +104,13 @@ def test_hooks_fire(where, kind):
     assert calls == [module]
 
 
+def test_residual_stream_in_the_models_own_type_is_kept():
+    model = _model(d=256, depth=4)
+    model.residual_in_fp32 = False
+    _, launches = _one_token(model)
+    assert launches > 2
+
+
 def test_transposed_weight_is_read_as_the_tensor_says():
     model = _model()
     _one_token(model)

@@ -138,3 +138,9 @@ def test_fewer_layers_than_it_was_built_with():
     model.layer_norms = model.layer_norms[:1]
     assert len(model._token_operands()[2]) == 1
     assert _model(expansion=1.5)._token_operands() is None
+
+
+def test_residual_stream_in_the_models_own_type():
+    model = _model()
+    model.residual_in_fp32 = False
+    assert model._token_operands() is None
