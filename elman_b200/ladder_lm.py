@@ -16,6 +16,7 @@ import operator
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from . import _lib, _spectral, fused_ops
 from .mamba_gated_elman import MambaGatedElman, MambaGatedElmanCell
@@ -29,14 +30,22 @@ _DTYPE = operator.attrgetter("dtype")
 _DATA_PTR = torch.Tensor.data_ptr
 _module = nn.modules.module
 
+_LEVELS = {0: StockElman, 1: MambaGatedElman, 4: LowRankElman, 5: PureLowRankElman,
+           32: E32NoPresilu, 33: E33SelfGate, 57: E57LearnedRadius}
+
 
 def _runs_only(module, cls):
     """Calling `module` is cls.forward and nothing else: no subclass, no hook, no forward of its own."""
     return (type(module) is cls and not module._forward_hooks and not module._forward_pre_hooks
             and "forward" not in module.__dict__)
 
-_LEVELS = {0: StockElman, 1: MambaGatedElman, 4: LowRankElman, 5: PureLowRankElman,
-           32: E32NoPresilu, 33: E33SelfGate, 57: E57LearnedRadius}
+
+def _transformed():
+    """True where a call is more than its values: inside a functorch transform (vmap, grad, jvp), a level
+    of forward-mode differentiation, a trace or a compilation.  None of them sees a kernel that is
+    launched beside the framework's dispatcher."""
+    return (torch._C._functorch.peek_interpreter_stack() is not None or forward_ad._current_level >= 0
+            or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling())
 
 
 def get_ladder_level(level):
@@ -225,9 +234,10 @@ class LadderLM(nn.Module):
         emb, norm, head = mods.get("embedding"), mods.get("norm"), mods.get("lm_head")
         # the layers' path calls the embedding, the layers, their cells and dropout modules; of the
         # others it reads the weights
-        if type(self) is not LadderLM or not self.fused_ops or not self.residual_in_fp32 \
-                or _module._global_forward_hooks or _module._global_forward_pre_hooks or not _runs_only(emb, nn.Embedding) \
-                or emb.max_norm is not None or type(norm) is not nn.RMSNorm or type(head) is not nn.Linear:
+        if type(self) is not LadderLM or not self.fused_ops or not self.residual_in_fp32 or _transformed() \
+                or _module._global_forward_hooks or _module._global_forward_pre_hooks \
+                or not _runs_only(emb, nn.Embedding) or emb.max_norm is not None \
+                or type(norm) is not nn.RMSNorm or type(head) is not nn.Linear:
             return None
         params = [emb._parameters.get("weight")]
         eps, cells = norm.eps, []

@@ -152,3 +152,13 @@ def test_model_is_copied_and_saved_after_a_token():
     torch.save(model, buffer)
     buffer.seek(0)
     assert torch.equal(_one_token(torch.load(buffer, weights_only=False))[0], want)
+
+
+def test_forward_mode_is_refused_and_not_dropped():
+    """The layers' autograd function has no forward derivative and says so."""
+    model = _model()
+    states = [torch.zeros(3, 64, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    with torch.no_grad(), torch.autograd.forward_ad.dual_level():
+        states[0] = torch.autograd.forward_ad.make_dual(states[0], torch.ones_like(states[0]))
+        with pytest.raises(RuntimeError):
+            model(_tokens(), prev_hiddens=states)

@@ -144,3 +144,18 @@ def test_residual_stream_in_the_models_own_type():
     model = _model()
     model.residual_in_fp32 = False
     assert model._token_operands() is None
+
+
+def test_transforms_of_the_call():
+    model, seen = _model(), []
+
+    def look(x):
+        seen.append(model._token_operands())
+        return x
+
+    torch.func.vmap(look)(torch.zeros(2))
+    with torch.autograd.forward_ad.dual_level():
+        look(None)
+    torch.jit.trace(look, torch.zeros(2), check_trace=False)
+    assert seen == [None, None, None]
+    assert model._token_operands() is not None
