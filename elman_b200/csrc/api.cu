@@ -1644,7 +1644,7 @@ int elman_e1_lm_token(int dtype, int depth, int B, int d, int vocab, const long 
   LmTokenArgs a{depth, B, d, vocab, tokens, embedding, layers, norm, head, eps, target_radius,
                 spectral_eps, logits, workspace};
   const int rc = lm_token(a, (cudaStream_t)stream);
-  if (rc == ELMAN_ERR_UNSUPPORTED) return set_error(rc, "an operand is not 16-byte aligned");
+  if (rc == ELMAN_ERR_UNSUPPORTED) return set_error(rc, "an operand is not aligned as elman_e1_lm_token asks");
   return rc;
 }
 

@@ -755,7 +755,9 @@ int lm_token(const LmTokenArgs& a, cudaStream_t stream) {
   p.status = device_status_ptr();
   p.spin_limit = options().spin_limit;
   p.stall_layer = (int)options().test_stall_step;
+  // read 16 bytes at a time; in feature pairs
   uintptr_t wide = (uintptr_t)a.embedding | (uintptr_t)a.norm | (uintptr_t)a.head | (uintptr_t)ws;
+  uintptr_t narrow = 0;
   q.d = a.d; q.NC = sp.NC; q.R = sp.R; q.groups = sp.groups;
   q.target = a.target; q.eps = a.spectral_eps;
   q.exchange_stride = ex_floats;
@@ -771,10 +773,11 @@ int lm_token(const LmTokenArgs& a, cudaStream_t stream) {
       if (r[k] == nullptr) return set_error(ELMAN_ERR_ARG, "layer %d: pointer %d is NULL", l, k);
     if (r[8] == nullptr) return set_error(ELMAN_ERR_ARG, "layer %d: pointer 8 is NULL", l);
     wide |= (uintptr_t)r[0] | (uintptr_t)r[1] | (uintptr_t)r[2] | (uintptr_t)r[3] | (uintptr_t)r[5] | (uintptr_t)r[7];
+    narrow |= (uintptr_t)r[4] | (uintptr_t)r[8];
     o.scale = r[6] != nullptr ? scales + l : nullptr;
     if (r[6] != nullptr) normed[n_normed++] = l;
   }
-  if ((wide & 15) != 0) return ELMAN_ERR_UNSUPPORTED;
+  if ((wide & 15) != 0 || (narrow & 3) != 0) return ELMAN_ERR_UNSUPPORTED;
   LmTokenKernel kern = pick_token_kernel(a.d, a.B);
   if (kern == nullptr) return ELMAN_ERR_UNSUPPORTED;
   ELMAN_CUDA_CHECK(cudaMemsetAsync(ws, 0xFF, act + exb + 256, stream));

@@ -220,7 +220,7 @@ class LadderLM(nn.Module):
                 eps, _spectral.TARGET_RADIUS, _spectral.EPS,
                 logits.data_ptr(), ws.data_ptr(), ws.numel(),
                 torch.cuda.current_stream(device).cuda_stream)
-        if rc == _lib.ELMAN_ERR_UNSUPPORTED:     # an operand off its 16-byte boundary
+        if rc == _lib.ELMAN_ERR_UNSUPPORTED:     # an operand off its boundary
             return None
         _lib.check(rc, "elman_e1_lm_token")
         return logits, list(hiddens.unbind(0))

@@ -546,7 +546,8 @@ int elman_adamw_step(int dtype, long n, void* params, const void* grads, void* e
  * pointers per layer: norm [d], in_proj [2d,d], W_x [d,d], W_h [d,d], b [d], out_proj [d,d],
  * u [d] (spectral normalisation's vector, advanced in place; NULL: W_h as it is),
  * h_prev [B,d] (NULL: zeros), h_out [B,d].  Outputs: h_out of every layer, logits [B,vocab].
- * Matrices, norms, embedding and h_prev must be 16-byte aligned.  A token outside [0, vocab) sets
+ * Matrices, norms, embedding and h_prev must be 16-byte aligned, b and h_out 4-byte aligned; for
+ * others ELMAN_ERR_UNSUPPORTED is returned and nothing is launched.  A token outside [0, vocab) sets
  * the device status word (detail 8 << 24 | 0xFFFFFE).
  */
 int elman_e1_lm_token_supported(int dtype, int depth, int B, int d, int vocab);

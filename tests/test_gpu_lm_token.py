@@ -3,6 +3,8 @@ the edges of its tiles: sequences around the 8-row tiles and the 32-row turns, w
 or a warp's K range partly filled, with and without carried states, with and without spectral
 normalisation.  Tolerance: the parity tests' bf16 2e-2 — both sides round activations to 8 bits six
 times per layer."""
+import ctypes
+
 import pytest
 import torch
 
@@ -73,3 +75,29 @@ def test_gives_up_when_a_block_stalls_and_recovers():
         code, detail = _lib.device_status(clear=True)
         assert code == 3 and detail >> 24 == 8
         assert torch.equal(model(tok), want)
+
+
+def test_bias_between_two_words_goes_layer_by_layer():
+    """Parameters packed into one flat buffer may start at any element; the kernel reads the bias in
+    pairs of features.  A state buffer of a C caller that starts there is refused."""
+    model = _model(64, 2, "none")
+    tok = torch.tensor([[3], [5]]).cuda()
+    with torch.no_grad():
+        model.layers[0].cell.b.normal_()
+        want = model(tok)
+        flat = torch.empty(65, dtype=torch.bfloat16, device="cuda")
+        flat[1:] = model.layers[0].cell.b
+        model.layers[0].cell.b.data = flat[1:]
+        before = _lib.launch_count()
+        got = model(tok)
+        assert _lib.launch_count() - before > 2
+    assert orc.rel_err(got.float().cpu(), want.float().cpu()) < TOL[torch.bfloat16]
+    lib, x = _lib.load(), torch.zeros(4096, dtype=torch.bfloat16, device="cuda")
+    ws = torch.empty(lib.elman_e1_lm_token_workspace(1, 1, 32), dtype=torch.uint8, device="cuda")
+    at = x.data_ptr()
+    for bias, h_out in ((at + 2, at), (at, at + 2)):
+        refs = (ctypes.c_void_p * 9)(at, at, at, at, bias, at, None, None, h_out)
+        before = _lib.launch_count()
+        rc = lib.elman_e1_lm_token(_lib.ELMAN_BF16, 1, 1, 32, 16, at, at, refs, at, at, 1e-6, 0.99, 1e-8,
+                                   at, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+        assert rc == _lib.ELMAN_ERR_UNSUPPORTED and _lib.launch_count() == before
