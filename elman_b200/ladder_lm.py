@@ -9,8 +9,8 @@ residual stream -> Elman layer) -> final add + norm -> tied linear head ->
 arguments that only concern other levels of the reference are accepted and
 ignored.
 """
+import array
 import contextlib
-import ctypes
 import operator
 
 import torch
@@ -25,10 +25,10 @@ from .siblings import E32NoPresilu, E33SelfGate, E57LearnedRadius, LowRankElman
 from .stock_elman import StockElman
 
 _NO_SWITCH = contextlib.nullcontext()
-_PLAIN_TENSORS = {torch.Tensor, nn.Parameter}
-_DTYPE = operator.attrgetter("dtype")
-_DATA_PTR = torch.Tensor.data_ptr
 _module = nn.modules.module
+_PLAIN_TENSORS = {torch.Tensor, nn.Parameter}
+_BF16 = {torch.bfloat16}
+_dtype_of = operator.attrgetter("dtype")
 
 _LEVELS = {0: StockElman, 1: MambaGatedElman, 4: LowRankElman, 5: PureLowRankElman,
            32: E32NoPresilu, 33: E33SelfGate, 57: E57LearnedRadius}
@@ -36,8 +36,19 @@ _LEVELS = {0: StockElman, 1: MambaGatedElman, 4: LowRankElman, 5: PureLowRankElm
 
 def _runs_only(module, cls):
     """Calling `module` is cls.forward and nothing else: no subclass, no hook, no forward of its own."""
-    return (type(module) is cls and not module._forward_hooks and not module._forward_pre_hooks
-            and "forward" not in module.__dict__)
+    if type(module) is not cls:
+        return False
+    own = module.__dict__
+    return not (own["_forward_hooks"] or own["_forward_pre_hooks"] or "forward" in own)
+
+
+def _all_like(tensors, device_index, sizes):
+    """Plain contiguous bf16 tensors of these sizes on one device: one pass per question, which is the
+    cheapest way to ask it of fifty tensors."""
+    return (_PLAIN_TENSORS.issuperset(map(type, tensors)) and set(map(_dtype_of, tensors)) == _BF16
+            and set(map(torch.Tensor.get_device, tensors)) == {device_index}
+            and all(map(torch.Tensor.is_contiguous, tensors))
+            and list(map(torch.Tensor.size, tensors)) == sizes)
 
 
 def _transformed():
@@ -193,37 +204,43 @@ class LadderLM(nn.Module):
         lib = _lib.load()
         if not lib.elman_e1_lm_token_supported(_lib.ELMAN_BF16, depth, B, d, V):
             return None
-        addresses = list(map(_DATA_PTR, params))
+        given = [h if h is None or h.is_contiguous() else h.contiguous() for h in prev_hiddens]
+        vectors = []
+        for cell, W_h in zip(cells, params[4::6]):
+            u = None
+            if cell.w_h_mode == "spectral_norm":
+                u = cell.__dict__.get("_spectral_u")
+                if u is None:
+                    u = _spectral.library_vector(cell, W_h)
+            vectors.append(u)
         hiddens = torch.empty(depth, B, d, dtype=torch.bfloat16, device=device)
-        h_out, h_bytes, shape = hiddens.data_ptr(), B * d * 2, (B, d)
-        keep, table = [], []
-        for i, (h, cell) in enumerate(zip(prev_hiddens, cells)):
-            table += addresses[1 + 6 * i:7 + 6 * i]
-            table.append(_spectral.library_vector(cell, params[4 + 6 * i]).data_ptr()
-                         if cell.w_h_mode == "spectral_norm" else None)
-            if h is not None:
-                if h.dtype is not torch.bfloat16 or h.device != device or h.shape != shape:
-                    return None
-                if not h.is_contiguous():
-                    h = h.contiguous()
-                    keep.append(h)
-                h = h.data_ptr()
-            table.append(h)
-            table.append(h_out + i * h_bytes)
+        states = hiddens.unbind(0)
+        row, shape = params[-2].shape, states[0].shape
+        us = [u for u in vectors if u is not None]
+        hs = [h for h in given if h is not None]
+        if (us or hs) and not _all_like(us + hs, device.index, [row] * len(us) + [shape] * len(hs)):
+            return None
+        addresses = list(map(torch.Tensor.data_ptr, params))
+        table, at = [], 1
+        for u, h, state in zip(vectors, given, states):
+            table += addresses[at:at + 6]
+            table += (0 if u is None else u.data_ptr(), 0 if h is None else h.data_ptr(), state.data_ptr())
+            at += 6
+        table = array.array("Q", table)
         tokens = inp.contiguous()
         logits = torch.empty(B, 1, V, dtype=torch.bfloat16, device=device)
         with torch.cuda.device(device) if torch.cuda.current_device() != device.index else _NO_SWITCH:
             ws = torch.empty(lib.elman_e1_lm_token_workspace(depth, B, d), dtype=torch.uint8, device=device)
             rc = lib.elman_e1_lm_token(
                 _lib.ELMAN_BF16, depth, B, d, V, tokens.data_ptr(), addresses[0],
-                (ctypes.c_void_p * len(table))(*table), addresses[-2], addresses[-1],
+                table.buffer_info()[0], addresses[-2], addresses[-1],
                 eps, _spectral.TARGET_RADIUS, _spectral.EPS,
                 logits.data_ptr(), ws.data_ptr(), ws.numel(),
                 torch.cuda.current_stream(device).cuda_stream)
         if rc == _lib.ELMAN_ERR_UNSUPPORTED:     # an operand off its boundary
             return None
         _lib.check(rc, "elman_e1_lm_token")
-        return logits, list(hiddens.unbind(0))
+        return logits, list(states)
 
     def _token_operands(self):
         """What the generation kernel reads: ([embedding, then per layer norm, in_proj, W_x, W_h, b,
@@ -247,30 +264,28 @@ class LadderLM(nn.Module):
         for layer, ln in zip(layers.values(), norms.values()):
             if not _runs_only(layer, MambaGatedElman) or layer.use_conv or not layer.fused:
                 return None
-            lm = layer._modules
-            drop = lm.get("dropout")      # its own switch decides, not the model's
-            if not _runs_only(drop, nn.Identity) and (not _runs_only(drop, nn.Dropout) or drop.training):
+            parts = layer._modules
+            drop, cell, w_in, w_out = map(parts.get, ("dropout", "cell", "in_proj", "out_proj"))
+            # (a dropout module's own switch decides, not the model's)
+            if not _runs_only(cell, MambaGatedElmanCell) or not (
+                    _runs_only(drop, nn.Identity) or (_runs_only(drop, nn.Dropout) and not drop.training)) \
+                    or type(w_in) is not nn.Linear or type(w_out) is not nn.Linear \
+                    or type(ln) is not nn.RMSNorm or ln.eps != eps:
                 return None
-            cell, w_in, w_out = lm.get("cell"), lm.get("in_proj"), lm.get("out_proj")
-            if not _runs_only(cell, MambaGatedElmanCell) or type(w_in) is not nn.Linear \
-                    or type(w_out) is not nn.Linear or type(ln) is not nn.RMSNorm or ln.eps != eps:
-                return None
-            cp = cell._parameters
-            params += (ln._parameters.get("weight"), w_in._parameters.get("weight"), cp.get("W_x"),
-                       cp.get("W_h"), cp.get("b"), w_out._parameters.get("weight"))
+            own = cell._parameters.get
+            params += (ln._parameters.get("weight"), w_in._parameters.get("weight"), own("W_x"), own("W_h"),
+                       own("b"), w_out._parameters.get("weight"))
             cells.append(cell)
         params += (norm._parameters.get("weight"), head._parameters.get("weight"))
-        if not _PLAIN_TENSORS.issuperset(map(type, params)) \
-                or set(map(_DTYPE, params)) != {torch.bfloat16} \
-                or len(set(map(torch.Tensor.get_device, params))) != 1 \
-                or not all(map(torch.Tensor.is_contiguous, params)):
+        if params[0] is None or params[-2] is None:
             return None
         # one width throughout; the vocabulary is what the tables hold
-        table, d = params[0].shape, params[-2].numel()
-        row, square = torch.Size((d,)), torch.Size((d, d))
-        want = [torch.Size((table[0], d))]
-        want += [row, torch.Size((2 * d, d)), square, square, row, square] * len(cells) + [row, want[0]]
-        if list(map(torch.Tensor.size, params)) != want:
+        d = params[-2].numel()
+        table, row, square = torch.Size((params[0].shape[0], d)), torch.Size((d,)), torch.Size((d, d))
+        want = [table]
+        want += [row, torch.Size((2 * d, d)), square, square, row, square] * len(cells)
+        want += [row, table]
+        if not _all_like(params, params[0].get_device(), want):
             return None
         return params, fused_ops.rmsnorm_eps(norm, torch.bfloat16), cells
 

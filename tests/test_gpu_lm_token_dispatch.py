@@ -162,3 +162,16 @@ def test_forward_mode_is_refused_and_not_dropped():
         states[0] = torch.autograd.forward_ad.make_dual(states[0], torch.ones_like(states[0]))
         with pytest.raises(RuntimeError):
             model(_tokens(), prev_hiddens=states)
+
+
+def test_vector_that_was_reset_is_drawn_again():
+    model = _model(r_h_mode="spectral_norm", r_h_init_gain=1.0)
+    _one_token(model)
+    states = [torch.full((3, 64), 0.5, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    with torch.no_grad():
+        want = model(_tokens(), prev_hiddens=states)
+        for layer in model.layers:
+            layer.cell._spectral_u = None
+        got = model(_tokens(), prev_hiddens=states)
+    assert all(layer.cell._spectral_u is not None for layer in model.layers)
+    assert orc.rel_err(got.float().cpu(), want.float().cpu()) < 0.1    # another start of three iterations
