@@ -220,6 +220,8 @@ class LadderLM(nn.Module):
         hs = [h for h in given if h is not None]
         if (us or hs) and not _all_like(us + hs, device.index, [row] * len(us) + [shape] * len(hs)):
             return None
+        if len(set(map(id, us))) != len(us):     # layers that share a cell advance its vector in turn
+            return None
         addresses = list(map(torch.Tensor.data_ptr, params))
         table, at = [], 1
         for u, h, state in zip(vectors, given, states):

@@ -164,6 +164,18 @@ def test_forward_mode_is_refused_and_not_dropped():
             model(_tokens(), prev_hiddens=states)
 
 
+def test_layers_that_share_a_cell_advance_its_vector_in_turn():
+    model = _model(r_h_mode="spectral_norm", r_h_init_gain=1.0)
+    model.layers[1] = model.layers[0]
+    u = nn.functional.normalize(torch.randn(64, device="cuda"), dim=0).bfloat16()
+    after = []
+    for run in (_layer_by_layer, lambda m: _one_token(m)[0]):
+        model.layers[0].cell._spectral_u = u.clone()
+        run(model)
+        after.append(model.layers[0].cell._spectral_u.float().cpu())
+    assert torch.equal(after[0], after[1])
+
+
 def test_vector_that_was_reset_is_drawn_again():
     model = _model(r_h_mode="spectral_norm", r_h_init_gain=1.0)
     _one_token(model)
