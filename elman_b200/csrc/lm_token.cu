@@ -110,6 +110,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) lm_token_kernel(const __grid_co
   __shared__ __align__(8) uint64_t landed[3];                 // in_proj, W_x, out_proj rows of a layer
   __shared__ int s_bad[2];
   __shared__ int s_abort;
+  __shared__ int s_sent[3];                                   // layer last sent for, by group
   extern __shared__ __align__(128) uint8_t lt_dyn[];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -142,7 +143,10 @@ __global__ void __launch_bounds__(LT_THREADS, 1) lm_token_kernel(const __grid_co
     if (l >= L || warp != RR_WARPS - 1) return;
     const LayerRefs& r = p.layer[l];
     const uint32_t bytes = (uint32_t)d * 2u;
-    if (lane == 0) ptx::mbar_arrive_expect_tx(&landed[group], (uint32_t)((group == 0 ? 2 : 1) * rows_here) * bytes);
+    if (lane == 0) {
+      s_sent[group] = l;
+      ptx::mbar_arrive_expect_tx(&landed[group], (uint32_t)((group == 0 ? 2 : 1) * rows_here) * bytes);
+    }
     __syncwarp();
     const int slot = group == 0 ? lane >> 4 : group + 1, row = lane & 15;
     if ((group == 0 || lane < 16) && row < rows_here) {
@@ -413,10 +417,16 @@ __global__ void __launch_bounds__(LT_THREADS, 1) lm_token_kernel(const __grid_co
       }
     }
   }
-  if (dead) {       // nothing may still be landing in this CTA's shared memory when it goes
+  if (dead) {
+    // Nothing may still be landing in this CTA's shared memory when it goes: the rows sent for last
+    // (a group's earlier ones had landed before these were sent for).  They come from this device's
+    // own memory and always arrive; the wait's time limit is its bound.
+    settle_norm();
     __syncthreads();
-    if (tid == 0)
-      for (int i = 0; i < 200; ++i) __nanosleep(1000);
+    if (tid < 3) {
+      int none = 0;
+      ptx::mbar_wait(&landed[tid], (uint32_t)s_sent[tid] & 1u, 1L << 40, &none);
+    }
     __syncthreads();
     return;
   }
