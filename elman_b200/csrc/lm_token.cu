@@ -37,6 +37,10 @@ namespace elman {
 namespace {
 
 constexpr int LT_MAX_LAYERS = 32;
+// The dynamic shared memory of the two kernels depends on the sizes, the limit they are launched under
+// must not: it belongs to the kernel, and another thread may set it between this one's setting and
+// launch.  So every call sets the same limit (the token kernel keeps 2 KB for its static arrays).
+constexpr int LT_SMEM_LIMIT = 225 * 1024, SP_SMEM_LIMIT = 220 * 1024;
 constexpr int LT_MAX_ROWS = 64;
 constexpr int LT_THREADS = 256;
 
@@ -694,7 +698,7 @@ bool spectral_plan(int L, int d, SpectralPlan* out) {
     if (groups < 1) return false;
     const size_t smem = ((size_t)d + (size_t)groups * d + (NC * R + 3) / 4 * 4 + (R + 3) / 4 * 4) * 4 +
                         (size_t)R * d * 2;
-    if (smem > 220 * 1024) continue;
+    if (smem > SP_SMEM_LIMIT) continue;
     *out = {m, NC, R, groups, smem};
     return true;
   }
@@ -730,7 +734,7 @@ bool lm_token_supported(int dtype, int L, int B, int d, int V) {
   if (L < 1 || L > LT_MAX_LAYERS || B < 1 || B > LT_MAX_ROWS || V < 1) return false;
   SpectralPlan sp;
   return d >= 32 && (d & 7) == 0 && d <= 1536 && (d + LT_R - 1) / LT_R <= rec_reg_sms() &&
-         lt_smem(d, token_tiles(B)) + 2048 <= 227 * 1024 && spectral_plan(L, d, &sp);
+         lt_smem(d, token_tiles(B)) <= LT_SMEM_LIMIT && spectral_plan(L, d, &sp);
 }
 
 // Everything that starts out as "not there yet", in one piece: three activation buffers per layer,
@@ -805,7 +809,7 @@ int lm_token(const LmTokenArgs& a, cudaStream_t stream) {
       q.W[j] = (const bf16*)r[3]; q.u[j] = (bf16*)const_cast<void*>(r[6]); q.scale[j] = scales + normed[i + j];
     }
     q.exchange = (float*)(ws + act) + (size_t)i * ex_floats;
-    ELMAN_CUDA_CHECK(cudaFuncSetAttribute(spectral_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp.smem));
+    ELMAN_CUDA_CHECK(cudaFuncSetAttribute(spectral_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SP_SMEM_LIMIT));
     cfg.gridDim = dim3(m * sp.NC);
     cfg.blockDim = dim3(SP_THREADS);
     cfg.dynamicSmemBytes = sp.smem;
@@ -815,7 +819,7 @@ int lm_token(const LmTokenArgs& a, cudaStream_t stream) {
   cfg.gridDim = dim3((a.d + LT_R - 1) / LT_R);
   cfg.blockDim = dim3(LT_THREADS);
   cfg.dynamicSmemBytes = lt_smem(a.d, token_tiles(a.B));
-  ELMAN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
+  ELMAN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_SMEM_LIMIT));
   ELMAN_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, (const LmTokenParams)p));
   count_launch(true);
   return ELMAN_OK;

@@ -4,6 +4,7 @@ or a warp's K range partly filled, with and without carried states, with and wit
 normalisation.  Tolerance: the parity tests' bf16 2e-2 — both sides round activations to 8 bits six
 times per layer."""
 import ctypes
+import threading
 
 import pytest
 import torch
@@ -101,3 +102,31 @@ def test_bias_between_two_words_goes_layer_by_layer():
         rc = lib.elman_e1_lm_token(_lib.ELMAN_BF16, 1, 1, 32, 16, at, at, refs, at, at, 1e-6, 0.99, 1e-8,
                                    at, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
         assert rc == _lib.ELMAN_ERR_UNSUPPORTED and _lib.launch_count() == before
+
+
+def test_two_threads_at_two_widths():
+    """Widths that share the kernels and differ in the shared memory they need: neither thread's launch
+    depends on what the other one last asked for."""
+    models = [_model(d, 2, "spectral_norm") for d in (1032, 1272)]
+    tok = torch.tensor([[3]]).cuda()
+    with torch.no_grad():
+        for m in models:
+            m(tok)
+    torch.cuda.synchronize()
+    errors = []
+
+    def generate(model):
+        try:
+            with torch.no_grad(), torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(400):
+                    model(tok)
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=generate, args=(m,)) for m in models]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors and _lib.device_status()[0] == 0
