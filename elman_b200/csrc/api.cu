@@ -37,6 +37,24 @@ void count_launch(bool tensor_core) {
   if (tensor_core) g_tc_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
+bool fits_together(const void* kernel, const cudaLaunchConfig_t& launch) {
+  const long blocks = (long)launch.gridDim.x * launch.gridDim.y * launch.gridDim.z;
+  const long limit = options().test_resident_blocks;
+  if (limit > 0 && blocks > limit) return false;
+  cudaLaunchConfig_t cfg = launch;       // blocks by themselves: clusters of one
+  cudaLaunchAttribute one;
+  one.id = cudaLaunchAttributeClusterDimension;
+  one.val.clusterDim.x = one.val.clusterDim.y = one.val.clusterDim.z = 1;
+  cfg.attrs = &one;
+  cfg.numAttrs = 1;
+  int fit = 0;
+  if (cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return blocks <= fit;
+}
+
 // One host-mapped status word per device, created on first use.
 static constexpr int kMaxDevices = 64;
 static int* g_status_host[kMaxDevices] = {nullptr};
@@ -248,7 +266,8 @@ static int run_rec_fwd(int dtype, int T, int B, int d, const void* W, const void
   a.compact = compact;
   if (reg_ok(dtype, T, B, d, compact)) {
     const int rc = rec_fwd_reg(a, st);
-    if (rc != ELMAN_ERR_UNSUPPORTED) return rc;   // an unaligned operand: nothing was launched
+    // an unaligned operand, or more blocks than fit together in this context: nothing was launched
+    if (rc != ELMAN_ERR_UNSUPPORTED) return rc;
   }
   if (dense_tc_ok(dtype, T, B, d, 0)) {
     // a plan that was co-resident when it was made may not be at launch time (another
@@ -335,6 +354,7 @@ int elman_b200_set_option(const char* name, long value) {
   else if (!strcmp(name, "rec_fin_groups")) o.rec_fin_groups = value;
   else if (!strcmp(name, "gemm_persistent")) o.gemm_persistent = value;
   else if (!strcmp(name, "gemm_pair")) o.gemm_pair = value;
+  else if (!strcmp(name, "test_resident_blocks")) o.test_resident_blocks = value;
   else if (!strcmp(name, "test_stall_step")) o.test_stall_step = value;
   else if (!strcmp(name, "rec_replicas")) o.rec_replicas = value;
   else if (!strcmp(name, "rec_group_cap")) o.rec_group_cap = value;
@@ -359,6 +379,7 @@ long elman_b200_get_option(const char* name) {
   if (!strcmp(name, "rec_fin_groups")) return o.rec_fin_groups;
   if (!strcmp(name, "gemm_persistent")) return o.gemm_persistent;
   if (!strcmp(name, "gemm_pair")) return o.gemm_pair;
+  if (!strcmp(name, "test_resident_blocks")) return o.test_resident_blocks;
   if (!strcmp(name, "test_stall_step")) return o.test_stall_step;
   if (!strcmp(name, "rec_replicas")) return o.rec_replicas;
   if (!strcmp(name, "rec_group_cap")) return o.rec_group_cap;
@@ -1644,7 +1665,8 @@ int elman_e1_lm_token(int dtype, int depth, int B, int d, int vocab, const long 
   LmTokenArgs a{depth, B, d, vocab, tokens, embedding, layers, norm, head, eps, target_radius,
                 spectral_eps, logits, workspace};
   const int rc = lm_token(a, (cudaStream_t)stream);
-  if (rc == ELMAN_ERR_UNSUPPORTED) return set_error(rc, "an operand is not aligned as elman_e1_lm_token asks");
+  if (rc == ELMAN_ERR_UNSUPPORTED) return set_error(rc, "an operand is not aligned as elman_e1_lm_token asks, or its "
+                                                          "blocks do not fit on the device together");
   return rc;
 }
 

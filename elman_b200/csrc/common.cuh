@@ -49,6 +49,7 @@ struct Options {
   long rec_trace = 0;
   long rec_mma_warps = 0;
   long rec_reg = 0;            // 0 auto, 1 never: the recurrence with W in registers
+  long test_resident_blocks = 0;   // test hook: the most blocks that fit on the device together (0: ask)
   long rec_direct_publish = 0;
   long rec_w_tmem = 0;
   long gemm_persistent = 0;    // 0 auto, 1 never, 2 always: the persistent 128x256 GEMM kernel
@@ -67,6 +68,23 @@ void count_launch(bool tensor_core);
 
 // Host-visible status word of the current device (mapped pinned memory).
 // Device code writes a non-zero code there when a bounded wait gives up.
+// Launches whose blocks wait for one another.  `fits_together`: all of this launch's blocks can be
+// resident at once on the current device as this context sees it (the kernel's shared-memory limit is
+// set; option test_resident_blocks stands in for a context with less room).  `launch_together`:
+// ELMAN_ERR_UNSUPPORTED, with nothing launched, where the runtime finds that a cooperative launch
+// does not fit.
+bool fits_together(const void* kernel, const cudaLaunchConfig_t& cfg);
+template <typename P>
+int launch_together(void (*kernel)(P), const cudaLaunchConfig_t& cfg, const P& params) {
+  const cudaError_t rc = cudaLaunchKernelEx(&cfg, kernel, params);
+  if (rc == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    return ELMAN_ERR_UNSUPPORTED;
+  }
+  ELMAN_CUDA_CHECK(rc);
+  return ELMAN_OK;
+}
+
 int* device_status_ptr();   // device-side alias, or nullptr if unavailable
 
 // kernel ids recorded in the status word

@@ -725,6 +725,12 @@ LmTokenKernel pick_token_kernel(int d, int B) {
   return nullptr;
 }
 
+// Behind a power iteration, which has advanced its vectors, nothing may start over.
+int too_late(int rc) {
+  return rc != ELMAN_ERR_UNSUPPORTED
+             ? rc : set_error(ELMAN_ERR_CUDA, "a cooperative launch was refused behind the power iterations");
+}
+
 size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
 }  // namespace
@@ -794,14 +800,27 @@ int lm_token(const LmTokenArgs& a, cudaStream_t stream) {
   if ((wide & 15) != 0 || (narrow & 3) != 0) return ELMAN_ERR_UNSUPPORTED;
   LmTokenKernel kern = pick_token_kernel(a.d, a.B);
   if (kern == nullptr) return ELMAN_ERR_UNSUPPORTED;
-  ELMAN_CUDA_CHECK(cudaMemsetAsync(ws, 0xFF, act + exb + 256, stream));
-  cudaLaunchConfig_t cfg{};
+  cudaLaunchConfig_t cfg{}, sp_cfg{};
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeCooperative;   // the CTAs of either launch wait for one another
   attr.val.cooperative = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  cfg.stream = stream;
+  cfg.attrs = sp_cfg.attrs = &attr;
+  cfg.numAttrs = sp_cfg.numAttrs = 1;
+  cfg.stream = sp_cfg.stream = stream;
+  cfg.gridDim = dim3((a.d + LT_R - 1) / LT_R);
+  cfg.blockDim = dim3(LT_THREADS);
+  cfg.dynamicSmemBytes = lt_smem(a.d, token_tiles(a.B));
+  sp_cfg.gridDim = dim3((n_normed < sp.per_launch ? n_normed : sp.per_launch) * sp.NC);
+  sp_cfg.blockDim = dim3(SP_THREADS);
+  sp_cfg.dynamicSmemBytes = sp.smem;
+  ELMAN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_SMEM_LIMIT));
+  if (!fits_together((const void*)kern, cfg)) return ELMAN_ERR_UNSUPPORTED;
+  if (n_normed > 0) {
+    ELMAN_CUDA_CHECK(cudaFuncSetAttribute(spectral_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          SP_SMEM_LIMIT));
+    if (!fits_together((const void*)spectral_many_kernel, sp_cfg)) return ELMAN_ERR_UNSUPPORTED;
+  }
+  ELMAN_CUDA_CHECK(cudaMemsetAsync(ws, 0xFF, act + exb + 256, stream));
   for (int i = 0; i < n_normed; i += sp.per_launch) {
     const int m = n_normed - i < sp.per_launch ? n_normed - i : sp.per_launch;
     for (int j = 0; j < m; ++j) {
@@ -809,18 +828,13 @@ int lm_token(const LmTokenArgs& a, cudaStream_t stream) {
       q.W[j] = (const bf16*)r[3]; q.u[j] = (bf16*)const_cast<void*>(r[6]); q.scale[j] = scales + normed[i + j];
     }
     q.exchange = (float*)(ws + act) + (size_t)i * ex_floats;
-    ELMAN_CUDA_CHECK(cudaFuncSetAttribute(spectral_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SP_SMEM_LIMIT));
-    cfg.gridDim = dim3(m * sp.NC);
-    cfg.blockDim = dim3(SP_THREADS);
-    cfg.dynamicSmemBytes = sp.smem;
-    ELMAN_CUDA_CHECK(cudaLaunchKernelEx(&cfg, spectral_many_kernel, (const SpectralManyParams)q));
+    sp_cfg.gridDim = dim3(m * sp.NC);
+    const int rc = launch_together(spectral_many_kernel, sp_cfg, q);
+    if (rc != ELMAN_OK) return i == 0 ? rc : too_late(rc);
     count_launch(false);
   }
-  cfg.gridDim = dim3((a.d + LT_R - 1) / LT_R);
-  cfg.blockDim = dim3(LT_THREADS);
-  cfg.dynamicSmemBytes = lt_smem(a.d, token_tiles(a.B));
-  ELMAN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_SMEM_LIMIT));
-  ELMAN_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, (const LmTokenParams)p));
+  const int rc = launch_together(kern, cfg, p);
+  if (rc != ELMAN_OK) return n_normed == 0 ? rc : too_late(rc);
   count_launch(true);
   return ELMAN_OK;
 }

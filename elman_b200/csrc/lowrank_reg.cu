@@ -91,6 +91,18 @@ int lowrank_reg(const LowRankRegArgs& a, cudaStream_t stream) {
   // 2.67 with no wait, 2.33 with these, 2.68 with 900 and 1200.
   p.hold = 600;
   p.hold_q = 600;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(((a.B < pl.rows ? a.B : pl.rows) + 8 * pl.nt - 1) / (8 * pl.nt) * pl.cpg);
+  cfg.blockDim = dim3(RR_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  // the runtime's guarantee that the CTAs, which wait for one another, are resident together
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeCooperative;
+  attr.val.cooperative = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (!fits_together((const void*)kern, cfg)) return ELMAN_ERR_UNSUPPORTED;
   const size_t slot = (size_t)a.B * a.d * sizeof(bf16), q_slot = (size_t)a.B * a.rq * sizeof(bf16);
   ELMAN_CUDA_CHECK(cudaMemsetAsync(a.sync, 0, 4, stream));
   ELMAN_CUDA_CHECK(cudaMemsetAsync((char*)a.state + (bwd ? 0 : slot), 0xFF, a.T * slot, stream));
@@ -99,18 +111,8 @@ int lowrank_reg(const LowRankRegArgs& a, cudaStream_t stream) {
     p.b_lo = b;
     p.b_hi = b + pl.rows < a.B ? b + pl.rows : a.B;
     const int groups = (p.b_hi - b + 8 * pl.nt - 1) / (8 * pl.nt);
-    cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(groups * pl.cpg);
-    cfg.blockDim = dim3(RR_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    // the runtime's guarantee that the CTAs, which wait for one another, are resident together
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeCooperative;
-    attr.val.cooperative = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    ELMAN_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, (const LowRankRegParams)p));
+    ELMAN_RETURN_IF(launch_together(kern, cfg, p));
     count_launch(true);
   }
   const int rows = (a.B + 8 * pl.nt - 1) / (8 * pl.nt);

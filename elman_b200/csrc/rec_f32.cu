@@ -243,23 +243,25 @@ int f32_launch(bool bwd, RecF32Params& p, int* sync, cudaStream_t stream) {
   p.abort_word = sync;
   p.status = device_status_ptr();
   p.spin_limit = options().spin_limit;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((per < groups ? per : groups) * p.cpg);
+  cfg.blockDim = dim3(RR_THREADS);
+  cfg.stream = stream;
+  // the runtime's guarantee that the CTAs, which wait for one another, are resident together
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeCooperative;
+  attr.val.cooperative = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (!fits_together((const void*)kern, cfg)) return ELMAN_ERR_UNSUPPORTED;
   const size_t slot = (size_t)p.B * p.d * sizeof(float);
   ELMAN_CUDA_CHECK(cudaMemsetAsync(sync, 0, 4, stream));
   ELMAN_CUDA_CHECK(cudaMemsetAsync((char*)p.state + (bwd ? 0 : slot), 0xFF, (size_t)p.T * slot, stream));
   for (int g = 0; g < groups; g += per) {
     p.b_lo = g * F32_NG;
     p.b_hi = (g + per) * F32_NG < p.B ? (g + per) * F32_NG : p.B;
-    cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((p.b_hi - p.b_lo + F32_NG - 1) / F32_NG * p.cpg);
-    cfg.blockDim = dim3(RR_THREADS);
-    cfg.stream = stream;
-    // the runtime's guarantee that the CTAs, which wait for one another, are resident together
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeCooperative;
-    attr.val.cooperative = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    ELMAN_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, (const RecF32Params)p));
+    ELMAN_RETURN_IF(launch_together(kern, cfg, p));
     count_launch(false);
   }
   if (bwd && groups > 1) return fold_db_rows(p.db, p.d, groups, stream);

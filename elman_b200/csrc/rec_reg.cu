@@ -137,7 +137,7 @@ bool rr_enabled() {
          o.rec_trace == 0;
 }
 
-int rr_launch(bool bwd, const RecRegPlan& pl, RecRegParams& p, int* sync, cudaStream_t stream) {
+int rr_launch(bool bwd, const RecRegPlan& pl, RecRegParams& p, int* sync, int compact, cudaStream_t stream) {
   const bool turns = pl.turns > 0;
   RecRegKernel kern = turns ? (bwd ? rec_turns_bwd_kernel(pl.kb) : rec_turns_fwd_kernel(pl.kb))
                       : bwd ? rec_reg_bwd_kernel(pl.mt, pl.kb, pl.nt)
@@ -151,6 +151,21 @@ int rr_launch(bool bwd, const RecRegPlan& pl, RecRegParams& p, int* sync, cudaSt
   const size_t smem = turns ? rec_turns_smem(bwd, pl.mt) : rec_reg_smem(bwd, pl.mt, pl.nt);
   if (smem > 48 * 1024)
     ELMAN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // CTAs wait for one another.  A cooperative launch is the runtime's guarantee that they are
+  // resident together, whatever else runs.  Callers that overlap launches (ELMAN_FLAG_COMPACT) go
+  // without it, since it would hold a launch back until all of it fits at once: they run side by side
+  // only what fits side by side, by elman_b200_recurrence_blocks, which is 0 under 128 features.
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(pl.groups * pl.cpg);
+  cfg.blockDim = dim3(turns ? RR_TURN_THREADS : RR_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeCooperative;
+  attr.val.cooperative = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = compact && p.d >= RR_MIN_CONCURRENT_D ? 0 : 1;
+  if (!fits_together((const void*)kern, cfg)) return ELMAN_ERR_UNSUPPORTED;
   p.b_lo = 0; p.b_hi = p.B;
   p.cpg = pl.cpg;
   p.turns = pl.turns;
@@ -163,20 +178,7 @@ int rr_launch(bool bwd, const RecRegPlan& pl, RecRegParams& p, int* sync, cudaSt
   // every slot the kernel writes starts out as "not there yet"
   const size_t slot = (size_t)p.B * p.d * sizeof(bf16);
   ELMAN_CUDA_CHECK(cudaMemsetAsync((char*)p.state + (bwd ? 0 : slot), 0xFF, (size_t)p.T * slot, stream));
-  // CTAs wait for one another.  A cooperative launch is the runtime's guarantee that they are
-  // resident together; shapes under 128 features, which callers that overlap launches do not
-  // plan for (elman_b200_recurrence_blocks reports 0), ask for it.
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(pl.groups * pl.cpg);
-  cfg.blockDim = dim3(turns ? RR_TURN_THREADS : RR_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeCooperative;
-  attr.val.cooperative = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = p.d < RR_MIN_CONCURRENT_D ? 1 : 0;
-  ELMAN_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, (const RecRegParams)p));
+  ELMAN_RETURN_IF(launch_together(kern, cfg, p));
   count_launch(true);
   return ELMAN_OK;
 }
@@ -211,7 +213,7 @@ int rec_fwd_reg(const RecFwdArgs& a, cudaStream_t stream) {
   p.in0 = (const bf16*)a.pre; p.in1 = (const bf16*)a.g;
   p.self_gate = a.g == nullptr ? 1 : 0;
   p.state = (bf16*)a.h; p.out0 = (bf16*)a.v; p.out1 = (bf16*)a.y;
-  return rr_launch(false, pl, p, a.sync, stream);
+  return rr_launch(false, pl, p, a.sync, a.compact, stream);
 }
 
 int rec_bwd_reg(const RecBwdArgs& a, cudaStream_t stream) {
@@ -224,7 +226,7 @@ int rec_bwd_reg(const RecBwdArgs& a, cudaStream_t stream) {
   p.in0 = (const bf16*)(a.g != nullptr ? a.g : a.dy); p.in1 = (const bf16*)a.dy;
   p.in2 = (const bf16*)a.h; p.in3 = (const bf16*)a.v;
   p.state = (bf16*)a.dv; p.out0 = (bf16*)a.dg; p.db = a.db;
-  ELMAN_RETURN_IF(rr_launch(true, pl, p, a.sync, stream));
+  ELMAN_RETURN_IF(rr_launch(true, pl, p, a.sync, a.compact, stream));
   if (pl.groups > 1) return fold_db_rows(a.db, a.d, pl.groups, stream);
   return ELMAN_OK;
 }

@@ -89,6 +89,8 @@ int elman_b200_device_status(int* detail, int clear);
  *                    copy, n = at most n.  Results do not depend on it.
  *   "rec_group_cap"  widest batch group (16, 32 or 64 rows) the large-batch plan may form;
  *                    0 (default) = 64
+ *   "test_resident_blocks" test hook, 0 (default) = ask the device: the most thread blocks that fit
+ *                    on it together, for launches whose blocks wait for one another
  *   "test_stall_step" failure-detection test hook, -1 (default) = off.  With a value k >= 1
  *                    thread block 0 of the next tensor-core launches (recurrences: at time
  *                    step k; projection GEMMs: at K iteration k) waits for something that
@@ -209,10 +211,12 @@ int elman_e1_backward_carry(int dtype, int flags, int T, int B, int d,
 /*
  * Number of thread blocks the recurrence kernel of an E1/E0 call of this shape
  * keeps resident for the whole launch (each occupies one SM), or 0 when the shape
- * takes a cooperative-launch kernel, which the driver only starts when it fits.
- * The blocks of one launch wait for one another, so a caller that overlaps
- * several recurrence launches on different streams must keep the sum of their
- * resident blocks within the device's SM count (no counterpart in the reference).
+ * takes a kernel without a plan for overlapped launches.
+ * The blocks of one launch wait for one another.  Launches without
+ * ELMAN_FLAG_COMPACT are cooperative (or checked to fit): the driver starts them only
+ * when all of their blocks fit.  A caller that overlaps several launches WITH the flag
+ * on different streams must keep the sum of their resident blocks within the device's
+ * SM count (no counterpart in the reference).
  */
 int elman_b200_recurrence_blocks(int dtype, int flags, int T, int B, int d);
 

@@ -45,3 +45,54 @@ def test_unaligned_weights_take_another_kernel():
     a = H.mamba_gated_elman_forward(True, dev["x"], dev["z"], dev["h0"], dev["W_x"], dev["W_h"], dev["b"])
     b = H.mamba_gated_elman_forward(True, dev["x"], dev["z"], dev["h0"], dev["W_x"], W, dev["b"])
     assert orc.rel_err(b[1].float().cpu(), a[1].float().cpu()) < 1e-2
+
+
+def test_contexts_with_too_little_room_take_another_kernel():
+    """Where the blocks that wait for one another cannot all be resident, nothing of the launch runs and
+    the next kernel in line takes the call: dense in both precisions, low-rank, generation step."""
+    from elman_b200.ladder_lm import LadderLM
+    from _gpu_cases import oracle_e5, run_e5
+    inp, low = orc.make_e1_inputs(4, 5, 136, seed=1), orc.make_e5_inputs(3, 40, 136, 20, seed=2)
+    torch.manual_seed(3)
+    lm = LadderLM(vocab_size=64, dim=64, depth=2, level=1).cuda().bfloat16().eval()
+    tok = torch.tensor([[3]]).cuda()
+    for limit in (0, 1):
+        with option("test_resident_blocks", limit):
+            before = _lib.tc_launch_count()
+            got, ref = run_e1(inp, torch.bfloat16)
+            tc = _lib.tc_launch_count() - before
+            assert_close(errors(got, oracle_e1(ref)), TOL[torch.bfloat16], f"bf16, limit {limit}")
+            got, ref = run_e1(inp, torch.float32)
+            assert_close(errors(got, oracle_e1(ref)), TOL[torch.float32], f"fp32, limit {limit}")
+            got, ref = run_e5(low, torch.bfloat16)
+            assert_close(errors(got, oracle_e5(ref)), TOL[torch.bfloat16], f"low rank, limit {limit}")
+            before = _lib.launch_count()
+            with torch.no_grad():
+                lm(tok)
+            assert (_lib.launch_count() - before > 2) == (limit == 1)
+        if limit == 0:
+            free = tc
+    assert tc == free - 2, "both recurrences should have left the register kernel"
+    assert _lib.device_status()[0] == 0
+
+
+def test_calls_on_two_streams_do_not_wait_for_each_others_blocks():
+    """Two calls whose blocks do not fit on the device together, at the same time."""
+    T, B, d = 40, 64, 952
+    calls = []
+    for seed in (1, 2):
+        inp = orc.make_e1_inputs(T, B, d, seed=seed)
+        dev = {k: v.to(torch.bfloat16).cuda() for k, v in inp.items()}
+        args = (True, dev["x"], dev["z"], dev["h0"], dev["W_x"], dev["W_h"], dev["b"])
+        calls.append((torch.cuda.Stream(), args, H.mamba_gated_elman_forward(*args)))
+    assert 2 * H.recurrence_blocks(torch.bfloat16, T, B, d) > 148
+    torch.cuda.synchronize()
+    outs = [[], []]
+    for _ in range(20):
+        for i, (stream, args, _) in enumerate(calls):
+            with torch.cuda.stream(stream):
+                outs[i].append(H.mamba_gated_elman_forward(*args))
+    torch.cuda.synchronize()
+    assert _lib.device_status()[0] == 0
+    for (_, _, want), got in zip(calls, outs):
+        assert all(torch.equal(a, b) for g in got for a, b in zip(g, want))
