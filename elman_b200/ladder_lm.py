@@ -204,7 +204,6 @@ class LadderLM(nn.Module):
         lib = _lib.load()
         if not lib.elman_e1_lm_token_supported(_lib.ELMAN_BF16, depth, B, d, V):
             return None
-        given = [h if h is None or h.is_contiguous() else h.contiguous() for h in prev_hiddens]
         vectors = []
         for cell, W_h in zip(cells, params[4::6]):
             u = None
@@ -213,21 +212,23 @@ class LadderLM(nn.Module):
                 if u is None:
                     u = _spectral.library_vector(cell, W_h)
             vectors.append(u)
-        hiddens = torch.empty(depth, B, d, dtype=torch.bfloat16, device=device)
-        states = hiddens.unbind(0)
-        row, shape = params[-2].shape, states[0].shape
         us = [u for u in vectors if u is not None]
-        hs = [h for h in given if h is not None]
-        if (us or hs) and not _all_like(us + hs, device.index, [row] * len(us) + [shape] * len(hs)):
+        hs = [h for h in prev_hiddens if h is not None]
+        if not all(map(torch.Tensor.is_contiguous, hs)):
+            prev_hiddens = [h if h is None else h.contiguous() for h in prev_hiddens]
+            hs = [h for h in prev_hiddens if h is not None]
+        if (us or hs) and not _all_like(us + hs, device.index, [params[-2].shape] * len(us)
+                                        + [torch.Size((B, d))] * len(hs)):
             return None
         if len(set(map(id, us))) != len(us):     # layers that share a cell advance its vector in turn
             return None
+        hiddens = torch.empty(depth, B, d, dtype=torch.bfloat16, device=device)
         addresses = list(map(torch.Tensor.data_ptr, params))
-        table, at = [], 1
-        for u, h, state in zip(vectors, given, states):
+        table, at, state = [], 1, hiddens.data_ptr()
+        for u, h in zip(vectors, prev_hiddens):
             table += addresses[at:at + 6]
-            table += (0 if u is None else u.data_ptr(), 0 if h is None else h.data_ptr(), state.data_ptr())
-            at += 6
+            table += (0 if u is None else u.data_ptr(), 0 if h is None else h.data_ptr(), state)
+            at, state = at + 6, state + 2 * B * d
         table = array.array("Q", table)
         tokens = inp.contiguous()
         logits = torch.empty(B, 1, V, dtype=torch.bfloat16, device=device)
@@ -238,11 +239,11 @@ class LadderLM(nn.Module):
                 table.buffer_info()[0], addresses[-2], addresses[-1],
                 eps, _spectral.TARGET_RADIUS, _spectral.EPS,
                 logits.data_ptr(), ws.data_ptr(), ws.numel(),
-                torch.cuda.current_stream(device).cuda_stream)
+                torch._C._cuda_getCurrentRawStream(device.index))
         if rc == _lib.ELMAN_ERR_UNSUPPORTED:     # an operand off its boundary
             return None
         _lib.check(rc, "elman_e1_lm_token")
-        return logits, list(states)
+        return logits, list(hiddens.unbind(0))
 
     def _token_operands(self):
         """What the generation kernel reads: ([embedding, then per layer norm, in_proj, W_x, W_h, b,
@@ -266,12 +267,12 @@ class LadderLM(nn.Module):
         for layer, ln in zip(layers.values(), norms.values()):
             if not _runs_only(layer, MambaGatedElman) or layer.use_conv or not layer.fused:
                 return None
-            parts = layer._modules
-            drop, cell, w_in, w_out = map(parts.get, ("dropout", "cell", "in_proj", "out_proj"))
+            parts = layer._modules.get
+            cell, drop, w_in, w_out = parts("cell"), parts("dropout"), parts("in_proj"), parts("out_proj")
             # (a dropout module's own switch decides, not the model's)
-            if not _runs_only(cell, MambaGatedElmanCell) or not (
-                    _runs_only(drop, nn.Identity) or (_runs_only(drop, nn.Dropout) and not drop.training)) \
-                    or type(w_in) is not nn.Linear or type(w_out) is not nn.Linear \
+            if not _runs_only(cell, MambaGatedElmanCell) \
+                    or not _runs_only(drop, nn.Dropout if type(drop) is nn.Dropout else nn.Identity) \
+                    or (type(drop) is nn.Dropout and drop.training) or type(w_in) is not nn.Linear or type(w_out) is not nn.Linear \
                     or type(ln) is not nn.RMSNorm or ln.eps != eps:
                 return None
             own = cell._parameters.get
