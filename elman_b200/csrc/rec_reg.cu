@@ -1,7 +1,5 @@
 // Plans and launches of the register-resident recurrence (rec_reg.cuh).
-#include <map>
-#include <mutex>
-#include <tuple>
+#include <limits.h>
 
 #include "rec_reg_table.cuh"
 
@@ -78,7 +76,7 @@ RecRegPlan pick_rec_reg_plan(int B, int d) {
 // Sets of batch groups, each on CTAs of its own and taking turns there, on at most `ctas` CTAs.
 // (Copies of the grid over shares of the batch: option rec_replicas limits them as it does those of
 // the TMEM kernel.)
-RecRegPlan turns_plan(int B, int d, int ctas) {
+RecRegPlan turns_plan(int T, int B, int d, int ctas) {
   RecRegPlan pl{};
   pl.kb = ((d + 31) / 32 + RR_WARPS - 1) / RR_WARPS;
   pl.ok = false;
@@ -94,7 +92,9 @@ RecRegPlan turns_plan(int B, int d, int ctas) {
   pl.turns = (groups + sets - 1) / sets;
   pl.groups = (groups + pl.turns - 1) / pl.turns;
   if (pl.turns == 1) pl.turns = 0;
-  pl.ok = pl.groups * pl.cpg <= rec_reg_sms();
+  // the kernel holds the bytes of a time slot and the number of turns in 32 bits
+  pl.ok = pl.groups * pl.cpg <= rec_reg_sms() && (long)B * d < (1L << 30) &&
+          (long)T * pl.turns <= INT_MAX - RR_AHEAD;
   return pl;
 }
 
@@ -104,8 +104,8 @@ RecRegPlan turns_plan(int B, int d, int ctas) {
 // d 1280 B 32, six layers, 20 / 40 CTAs 11.52 / 11.62; d 768 B 13, six layers, 12 / 24 CTAs 3.32 /
 // 3.23; d 256 B 32, four layers, 4 / 8 CTAs 1.64 / 1.54.  Where every group has its own CTAs this
 // is rec_reg_kernel; a plan with more CTAs than the fast one is of no use.
-RecRegPlan pick_compact_plan(int B, int d, const RecRegPlan& fast) {
-  const RecRegPlan pl = turns_plan(B, d, rec_reg_sms() / 6);
+RecRegPlan pick_compact_plan(int T, int B, int d, const RecRegPlan& fast) {
+  const RecRegPlan pl = turns_plan(T, B, d, rec_reg_sms() / 6);
   return pl.ok && pl.groups * pl.cpg <= fast.groups * fast.cpg ? pl : fast;
 }
 
@@ -123,8 +123,8 @@ RecRegPlan pick_compact_plan(int B, int d, const RecRegPlan& fast) {
 //   512  1280  10.7  10.1    9.15  9.60        256   952   350   235    3.51  3.77   (CUDA cores)
 RecRegPlan plan_for(int T, int B, int d, int compact) {
   const RecRegPlan fast = pick_rec_reg_plan(B, d);
-  if (fast.ok) return compact ? pick_compact_plan(B, d, fast) : fast;
-  RecRegPlan pl = turns_plan(B, d, rec_reg_sms());
+  if (fast.ok) return compact ? pick_compact_plan(T, B, d, fast) : fast;
+  RecRegPlan pl = turns_plan(T, B, d, rec_reg_sms());
   const bool slow = compact || B > 512 || (pl.kb > 6 && pl.turns > 6);
   if (pl.ok && slow && rec_tc_supported(T, B, d, 0) && rec_tc_supported(T, B, d, 1)) pl.ok = false;
   return pl;

@@ -87,3 +87,11 @@ def test_wait_that_runs_out_ends_the_launch():
         assert code == 3 and (detail >> 24) & 0xFF == kid
     got, _ = run_compact(inp)
     assert_close(errors(got, oracle_e1(ref)), TOL[torch.bfloat16], "after the give-up")
+
+
+def test_time_slots_of_2_gib_stay_with_the_kernel_that_counts_in_64_bits():
+    """(No launch: what the planner says.)"""
+    d = 136
+    fits = (2 ** 30 - 1) // d
+    assert H.recurrence_blocks(torch.bfloat16, 2, fits, d) > 0
+    assert H.recurrence_blocks(torch.bfloat16, 2, fits + 1, d) == 0
