@@ -20,7 +20,7 @@ LIBDIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIBDIR, "libelman_b200.so")
 SOURCES = ["api.cu", "gemm_simt.cu", "gemm_tc.cu", "rec_simt.cu", "rec_tc.cu", "rec_reg.cu", "rec_reg_fwd.cu", "rec_reg_bwd.cu", "rec_turns_fwd.cu",
            "rec_turns_bwd.cu", "rec_f32.cu", "gemm_f32.cu", "lowrank_reg.cu", "lowrank_reg_fwd.cu",
-           "lowrank_reg_bwd.cu", "lowrank_tc.cu", "extras.cu", "layer_ops.cu", "train_ops.cu", "spectral.cu", "lm_token.cu"]
+           "lowrank_reg_bwd.cu", "lowrank_split_fwd.cu", "lowrank_split_bwd.cu", "lowrank_tc.cu", "extras.cu", "layer_ops.cu", "train_ops.cu", "spectral.cu", "lm_token.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-std=c++17", "-lineinfo",

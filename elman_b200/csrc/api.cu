@@ -692,22 +692,22 @@ static bool lowrank_reg_ok(int dtype, int T, int B, int d, int r, int flags) {
 }
 static int run_lowrank_reg_fwd(int T, int B, int d, int r, const void* U, const void* V,
                                const void* pre, const void* gate, void* h, void* y, void* v, void* q,
-                               int rq, int* sync, cudaStream_t st) {
+                               void* q_low, int rq, int* sync, cudaStream_t st) {
   PhaseTimer timer(0, st);
   LowRankRegArgs a{};
   a.T = T; a.B = B; a.d = d; a.r = r; a.bwd = 0;
   a.A1 = V; a.a1_row = d; a.a1_k = 1;
   a.A2 = U; a.a2_row = r; a.a2_k = 1;
   a.in0 = pre; a.in1 = gate; a.state = h; a.out0 = v; a.out1 = y;
-  a.q = q; a.rq = rq; a.sync = sync;
+  a.q = q; a.q_low = q_low; a.rq = rq; a.sync = sync;
   return lowrank_reg(a, st);
 }
 // dVh [T+1,B,rp]: slots 1 .. T-1 come out of the recurrence (slot T belongs to the carried-in
 // gradient), slot 0 is one more product of B rows.
 static int run_lowrank_reg_bwd(int T, int B, int d, int r, const void* U, const void* V,
                                const void* gate, const void* dy, const void* h, const void* v,
-                               void* dv, void* dg, float* db, void* dVh, int rp, const void* Upad,
-                               int* sync, cudaStream_t st) {
+                               void* dv, void* dg, float* db, void* dVh, void* q_low, int rp,
+                               const void* Upad, int* sync, cudaStream_t st) {
   {
     PhaseTimer timer(1, st);
     LowRankRegArgs a{};
@@ -715,7 +715,7 @@ static int run_lowrank_reg_bwd(int T, int B, int d, int r, const void* U, const 
     a.A1 = U; a.a1_row = 1; a.a1_k = r;
     a.A2 = V; a.a2_row = 1; a.a2_k = d;
     a.in0 = gate; a.in1 = dy; a.in2 = h; a.in3 = v; a.state = dv; a.out0 = dg; a.db = db;
-    a.q = dVh; a.rq = rp; a.sync = sync;
+    a.q = dVh; a.q_low = q_low; a.rq = rp; a.sync = sync;
     ELMAN_RETURN_IF(lowrank_reg(a, st));
   }
   return gemm_nn(ELMAN_BF16, B, rp, d, dv, d, Upad, rp, nullptr, dVh, rp, 0, st);
@@ -807,9 +807,9 @@ int elman_e5_forward_flags(int dtype, int flags, int training, int T, int B, int
   ELMAN_RETURN_IF(proj_nt(dtype, TB, d, rp, w.Vx, rp, Ux, rp, b, w.pre, d, 0, st));
   ELMAN_RETURN_IF(proj_nt(dtype, TB, rp, d, x, d, Vz, d, nullptr, w.Vz, rp, 0, st));
   ELMAN_RETURN_IF(proj_nt(dtype, TB, d, rp, w.Vz, rp, Uz, rp, nullptr, w.gate, d, 0, st));
-  if (lowrank_reg_ok(dtype, T, B, d, r, flags)) {   // the rank vectors go where x V_x^T was
+  if (lowrank_reg_ok(dtype, T, B, d, r, flags)) {   // the rank vectors go where x V_x^T and x V_z^T were
     const int rc = run_lowrank_reg_fwd(T, B, d, r, U_h, V_h, w.pre, w.gate, h, output,
-                                       training ? v : nullptr, w.Vx, rp, w.sync, st);
+                                       training ? v : nullptr, w.Vx, w.Vz, rp, w.sync, st);
     if (rc != ELMAN_ERR_UNSUPPORTED) return rc;
   }
   if (use_tc(dtype) && lowrank_tc_supported(T, B, d, r, 0)) {
@@ -966,7 +966,7 @@ int elman_e5_backward_carry_flags(int dtype, int flags, int T, int B, int d, int
   int rec = ELMAN_ERR_UNSUPPORTED;
   if (lowrank_reg_ok(dtype, T, B, d, r, flags))
     rec = run_lowrank_reg_bwd(T, B, d, r, U_h, V_h, w.gate, d_output, h, v, w.dv, w.dg, w.db, w.dVh,
-                              rp, Uh, w.sync, st);
+                              w.dVx, rp, Uh, w.sync, st);   // (dVx is written behind the recurrence)
   const bool have_dVh = rec == ELMAN_OK;
   if (rec != ELMAN_OK && rec != ELMAN_ERR_UNSUPPORTED) return rec;
   if (!have_dVh) {
@@ -1026,13 +1026,14 @@ int elman_e5_backward_carry_flags(int dtype, int flags, int T, int B, int d, int
 // projection of x and with z as the gate input; the time-parallel part is E1's.
 
 struct E4FwdWs {
-  void* q; void* pre; float* tmp; int* sync; long long* trace; void* UP; void* VP;
+  void* q; void* q_low; void* pre; float* tmp; int* sync; long long* trace; void* UP; void* VP;
 };
 static size_t carve_e4_fwd(int dtype, int T, int B, int d, int r, void* ws, E4FwdWs* o) {
   Carver c(ws);
   size_t es = esize(dtype);
   o->pre = c.take((size_t)T * B * d * es);
   o->q = c.take((size_t)T * B * e5_rank_alloc(dtype, r) * es);   // rank vectors
+  o->q_low = c.take((size_t)T * B * e5_rank_alloc(dtype, r) * es);
   o->tmp = (float*)c.take((size_t)2 * B * r * sizeof(float));
   o->sync = (int*)c.take(rec_sync_bytes());
   o->trace = (long long*)c.take(kTraceBytes);
@@ -1073,7 +1074,7 @@ int elman_e4_forward(int dtype, int training, int T, int B, int d, int r, const 
   ELMAN_RETURN_IF(proj_nt(dtype, T * B, d, d, x, d, W_x, d, b, w.pre, d, 0, st));
   if (lowrank_reg_ok(dtype, T, B, d, r, 0)) {
     const int rc = run_lowrank_reg_fwd(T, B, d, r, U, V, w.pre, z, h, output, training ? v : nullptr,
-                                       w.q, e5_rank_run(dtype, r), w.sync, st);
+                                       w.q, w.q_low, e5_rank_run(dtype, r), w.sync, st);
     if (rc != ELMAN_ERR_UNSUPPORTED) return rc;
   }
   if (use_tc(dtype) && lowrank_tc_supported(T, B, d, r, 0)) {
@@ -1165,8 +1166,8 @@ int elman_e4_backward(int dtype, int T, int B, int d, int r, const void* W_x, co
   ELMAN_CUDA_CHECK(cudaMemsetAsync((char*)w.dv + (size_t)T * B * d * es, 0, (size_t)B * d * es, st));
   int rec = ELMAN_ERR_UNSUPPORTED;
   if (lowrank_reg_ok(dtype, T, B, d, r, 0))
-    rec = run_lowrank_reg_bwd(T, B, d, r, U, V, z, d_output, h, v, w.dv, dz, w.db, w.dVh, rp, Uh, w.sync,
-                              st);
+    rec = run_lowrank_reg_bwd(T, B, d, r, U, V, z, d_output, h, v, w.dv, dz, w.db, w.dVh, w.Vh, rp, Uh,
+                              w.sync, st);   // (Vh is written behind the recurrence)
   const bool have_dVh = rec == ELMAN_OK;
   if (rec != ELMAN_OK && rec != ELMAN_ERR_UNSUPPORTED) return rec;
   if (!have_dVh) {

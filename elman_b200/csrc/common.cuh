@@ -298,6 +298,7 @@ int rec_reg_sms();   // multiprocessors of the current device
 //   backward: in0 = gate, in1 = dy, in2 = h, in3 = v, state = dv [T+1,B,d] (slot T filled), out0 = dg,
 //             db fp32 [REC_MAX_DB_ROWS, d], A1 = U^T, A2 = V^T;  q [T+1,B,rq]: slot t receives U^T dv_t
 //             for t = T .. 1
+//   q_low     : scratch [T,B,rq] for the shapes whose rank vectors lowrank_tc.cu does not round to bf16
 // Factors are read through strides: element (row, k) of A at row * a_row + k * a_k.
 struct LowRankRegArgs {
   int T, B, d, r, bwd;
@@ -305,7 +306,7 @@ struct LowRankRegArgs {
   const void* A2; long a2_row, a2_k;
   const void* in0; const void* in1; const void* in2; const void* in3;
   void* state; void* out0; void* out1; float* db;
-  void* q; int rq;
+  void* q; void* q_low; int rq;
   int* sync;
 };
 bool lowrank_reg_supported(int T, int B, int d, int r);

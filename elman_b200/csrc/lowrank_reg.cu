@@ -18,9 +18,11 @@ struct LowRankRegPlan {
 // Measured, us per step forward / backward, against what ran before:
 //
 //    B    d    r   before                          this kernel
-//   32 1536  270   5.6  6.0  (one cluster, TMEM)   2.33 2.41
+//   32 1536  270   5.6  6.0  (one cluster, TMEM)   2.37 2.52
 //    8 1024  152   4.3  4.6  (one cluster, TMEM)   1.84 1.89
-//  128 1536  270   239  317  (CUDA cores)          4.9  6.9
+//  128 1536  270   239  317  (CUDA cores)          5.4  6.0   (one part of the rank vector: 4.6 6.7)
+//   48 1536  270             (CUDA cores)          2.98 3.12  (2.51 2.69)
+//    9 1000  130             (CUDA cores)          2.38 2.44  (2.13 2.19)
 LowRankRegPlan pick_lowrank_reg_plan(int B, int d, int r) {
   LowRankRegPlan best{};
   best.ok = false;
@@ -63,14 +65,16 @@ int lowrank_reg(const LowRankRegArgs& a, cudaStream_t stream) {
   const LowRankRegPlan pl = pick_lowrank_reg_plan(a.B, a.d, a.r);
   if (!pl.ok) return ELMAN_ERR_UNSUPPORTED;
   const bool bwd = a.bwd != 0;
-  const uintptr_t wide = (uintptr_t)a.state | (uintptr_t)a.q;
+  // the rank vector with the bits that the kernel which had this shape before kept
+  const bool split = !lowrank_tc_supported(a.T, a.B, a.d, a.r, a.bwd);
+  const uintptr_t wide = (uintptr_t)a.state | (uintptr_t)a.q | (uintptr_t)a.q_low;
   const uintptr_t narrow = (uintptr_t)a.in0 | (uintptr_t)a.in1 | (uintptr_t)a.in2 | (uintptr_t)a.in3 |
                            (uintptr_t)a.out0 | (uintptr_t)a.out1;
   if ((wide & 15) != 0 || (narrow & 3) != 0 || (a.rq & 7) != 0) return ELMAN_ERR_UNSUPPORTED;
-  LowRankRegKernel kern = bwd ? lowrank_reg_bwd_kernel(pl.kb1, pl.kb2, pl.mt, pl.nt)
-                              : lowrank_reg_fwd_kernel(pl.kb1, pl.kb2, pl.mt, pl.nt);
+  LowRankRegKernel kern = (split ? (bwd ? lowrank_split_bwd_kernel : lowrank_split_fwd_kernel)
+                                 : (bwd ? lowrank_reg_bwd_kernel : lowrank_reg_fwd_kernel))(pl.kb1, pl.kb2, pl.mt, pl.nt);
   if (kern == nullptr) return ELMAN_ERR_UNSUPPORTED;
-  const size_t smem = lowrank_reg_smem(bwd, pl.mt, pl.nt);
+  const size_t smem = lowrank_reg_smem(bwd, pl.kb1, pl.kb2, pl.mt, pl.nt, split);
   if (smem > 48 * 1024)
     ELMAN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   LowRankRegParams p{};
@@ -81,7 +85,7 @@ int lowrank_reg(const LowRankRegArgs& a, cudaStream_t stream) {
   p.in0 = (const bf16*)a.in0; p.in1 = (const bf16*)a.in1;
   p.in2 = (const bf16*)a.in2; p.in3 = (const bf16*)a.in3;
   p.state = (bf16*)a.state; p.out0 = (bf16*)a.out0; p.out1 = (bf16*)a.out1; p.db = a.db;
-  p.q = (bf16*)a.q;
+  p.q = (bf16*)a.q; p.q_low = (bf16*)a.q_low;
   p.abort_word = a.sync;
   p.status = device_status_ptr();
   p.spin_limit = options().spin_limit;
@@ -107,6 +111,7 @@ int lowrank_reg(const LowRankRegArgs& a, cudaStream_t stream) {
   ELMAN_CUDA_CHECK(cudaMemsetAsync(a.sync, 0, 4, stream));
   ELMAN_CUDA_CHECK(cudaMemsetAsync((char*)a.state + (bwd ? 0 : slot), 0xFF, a.T * slot, stream));
   ELMAN_CUDA_CHECK(cudaMemsetAsync((char*)a.q + (bwd ? q_slot : 0), 0xFF, a.T * q_slot, stream));
+  if (split) ELMAN_CUDA_CHECK(cudaMemsetAsync(a.q_low, 0xFF, a.T * q_slot, stream));
   for (int b = 0; b < a.B; b += pl.rows) {
     p.b_lo = b;
     p.b_hi = b + pl.rows < a.B ? b + pl.rows : a.B;

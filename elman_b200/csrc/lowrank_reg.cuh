@@ -13,9 +13,19 @@
 // vectors are U^T dv of every step but the first, which the weight gradients need as well and
 // would otherwise compute again as a product over all T B rows.
 //
+// SPLIT: the rank vector in two bf16 parts, its rounded value and what the rounding left (16 bits of
+// mantissa together).  The cluster kernel (lowrank_tc.cu) rounds the vector to bf16 between the two
+// products, the CUDA-core kernel kept it in fp32; shapes that come from the latter (batches over 32,
+// widths that are no multiple of 128, ranks too large for one cluster) take this form.  Relative error of
+// h against 64 bits at T = 160, B = 128, d = 1536, r = 270: CUDA cores 2.748e-3, one part 2.930e-3, two
+// parts 2.747e-3.  The second part costs 0.3 to 0.5 us of a step.  It is stored first, so whoever has seen
+// the rounded value seldom waits for it.
+//
 // Bound, like the dense kernel's, by the chain: two L2 round trips per step.  Measured at B = 32,
 // d = 1536, r = 270: see lowrank_reg.cu.
 #pragma once
+
+#include <float.h>
 
 #include "rec_reg.cuh"
 
@@ -27,13 +37,21 @@ struct LowRankRegParams : RecRegParams {
   const bf16* A1; long a1_row, a1_k;   // first factor [r, d]:  element (row, k) at row*a1_row + k*a1_k
   const bf16* A2; long a2_row, a2_k;   // second factor [d, r]
   bf16* q;                      // rank vectors [slots][B][rq]; slot of a step = slot of its input state
+  bf16* q_low;                  // SPLIT: what rounding the entries of q to bf16 left, [T][B][rq]; slot = step
   int hold_q;                   // cycles from a CTA's last barrier to its first look at q
 };
 
 constexpr int LRR_PS1 = 20;     // row stride of the 16-row partial sums
 
-inline size_t lowrank_reg_smem(bool bwd, int mt, int nt) {
-  return rec_reg_smem(bwd, mt, nt) + (size_t)RR_WARPS * 8 * nt * LRR_PS1 * sizeof(float);
+// The first factor's fragments in shared memory instead of registers (8 KB1 of them): where both factors,
+// both parts of the rank vector and the accumulators would spill.
+__host__ __device__ constexpr bool lowrank_first_shared(int kb1, int kb2, int mt, bool split) {
+  return split && (mt * kb2 > 8 || (kb1 == 8 && mt * kb2 >= 6));
+}
+
+inline size_t lowrank_reg_smem(bool bwd, int kb1, int kb2, int mt, int nt, bool split) {
+  return rec_reg_smem(bwd, mt, nt) + (size_t)RR_WARPS * 8 * nt * LRR_PS1 * sizeof(float) +
+         (lowrank_first_shared(kb1, kb2, mt, split) ? (size_t)kb1 * 2 * RR_THREADS * sizeof(uint4) : 0);
 }
 
 namespace rr {
@@ -61,12 +79,19 @@ __device__ __forceinline__ void load_factor(uint32_t (&w)[KB][8], const bf16* A,
     }
 }
 
+// What rounding a pair to bf16 left of it, as bf16; nothing of an entry that is no finite number.
+__device__ __forceinline__ uint32_t rest(float2 v, uint32_t hi) {
+  const float2 h = unpack(hi);
+  return pack(fabsf(h.x) <= FLT_MAX ? v.x - h.x : 0.f, fabsf(h.y) <= FLT_MAX ? v.y - h.y : 0.f);
+}
+
 }  // namespace rr
 
-template <bool BWD, int KB1, int KB2, int MT, int NT>
+template <bool BWD, int KB1, int KB2, int MT, int NT, bool SPLIT>
 __global__ void __launch_bounds__(RR_THREADS, 1) lowrank_reg_kernel(const LowRankRegParams p) {
   constexpr int R = 16 * MT, NG = 8 * NT;
   constexpr int CH1 = NT == 1 ? 2 : 1, CH2 = MT * NT == 1 ? 2 : 1;
+  constexpr bool W1S = lowrank_first_shared(KB1, KB2, MT, SPLIT);
   typedef rr::Tail<BWD, R, NG> Tail;
   constexpr int PS = Tail::PS;
   extern __shared__ __align__(16) float part[];   // [2][warps][NG][PS], ring, [warps][NG][LRR_PS1]
@@ -84,9 +109,25 @@ __global__ void __launch_bounds__(RR_THREADS, 1) lowrank_reg_kernel(const LowRan
   const rr::KRange<KB2> k2(p.r16, warp, tq);
   uint32_t w1[1][KB1][8], w2[MT][KB2][8];
   rr::load_factor<KB1>(w1[0], p.A1, p.a1_row, p.a1_k, c * 16 + gq, p.r, k1, d);
+  // (every thread reads back its own)
+  uint4* const w1_s = reinterpret_cast<uint4*>(part + 2 * RR_WARPS * NG * PS +
+                                               RR_AHEAD * Tail::ITEMS * Tail::NIN * RR_THREADS +
+                                               RR_WARPS * NG * LRR_PS1) + tid;
+  if (W1S) {
+#pragma unroll
+    for (int kb = 0; kb < KB1; ++kb)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        w1_s[(kb * 2 + j) * RR_THREADS] = make_uint4(w1[0][kb][4 * j], w1[0][kb][4 * j + 1], w1[0][kb][4 * j + 2],
+                                                     w1[0][kb][4 * j + 3]);
+  }
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt)
     rr::load_factor<KB2>(w2[mt], p.A2, p.a2_row, p.a2_k, f0 + mt * 16 + gq, d, k2, p.r);
+  // a warp whose part of K is behind the rank has nothing to add, once and for all
+  const bool busy = !SPLIT || warp * (KB2 * 32) < p.r16;
+  if (!busy)
+    for (int i = lane; i < 2 * NG * PS; i += 32) part[(i / (NG * PS) * RR_WARPS + warp) * NG * PS + i % (NG * PS)] = 0.f;
   uint32_t h_off[NT], q_off[NT];
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) {
@@ -120,6 +161,7 @@ __global__ void __launch_bounds__(RR_THREADS, 1) lowrank_reg_kernel(const LowRan
     tail.premath(s);
     const long from = BWD ? T - s : s;            // time slot of the input state
     char* const q = reinterpret_cast<char*>(p.q) + from * q_slot;
+    char* const q_low = reinterpret_cast<char*>(p.q_low) + (long)s * q_slot;
     if (ranked) {
       // ---- my 16 entries of the rank vector ----
       const char* src = reinterpret_cast<const char*>(p.state) + from * slot;
@@ -128,6 +170,16 @@ __global__ void __launch_bounds__(RR_THREADS, 1) lowrank_reg_kernel(const LowRan
       rr::look(x, src, h_off);
       if (s > 0 && !rr::await(x, src, h_off, s == stall_step, p.spin_limit, p.abort_word)) give_up(0, s);
       __syncwarp();
+      if (W1S) {
+#pragma unroll
+        for (int kb = 0; kb < KB1; ++kb)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const uint4 v = w1_s[(kb * 2 + j) * RR_THREADS];
+            w1[0][kb][4 * j] = v.x; w1[0][kb][4 * j + 1] = v.y;
+            w1[0][kb][4 * j + 2] = v.z; w1[0][kb][4 * j + 3] = v.w;
+          }
+      }
       float acc[CH1][1][NT][4];
       rr::products(acc, w1, x);
       rr::put_partials(part1 + warp * NG * LRR_PS1, LRR_PS1, gq, tq, acc);
@@ -136,20 +188,31 @@ __global__ void __launch_bounds__(RR_THREADS, 1) lowrank_reg_kernel(const LowRan
       const int bad = s_bad[0][s & 1];
       if (mine1) {
         const float2 v = rr::gather_pair(part1 + n1 * LRR_PS1 + 2 * pair1, NG * LRR_PS1);
-        rr::st_relaxed_u32(q + q_mine, rr::pack(v.x, v.y));
+        const uint32_t hi = rr::pack(v.x, v.y);
+        if (SPLIT) rr::st_relaxed_u32(q_low + q_mine, rr::rest(v, hi));
+        rr::st_relaxed_u32(q + q_mine, hi);
       }
       if (bad) break;
     }
     // ---- my features from the whole rank vector ----
-    while (rr::cycles() - met < (uint32_t)p.hold_q) { }
-    uint4 x[NT][KB2];
-    rr::look(x, q, q_off);
-    if (!rr::await(x, q, q_off, false, p.spin_limit, p.abort_word)) give_up(1, s);
-    __syncwarp();
-    float acc[CH2][MT][NT][4];
-    rr::products(acc, w2, x);
     float* buf = part + (s & 1) * (RR_WARPS * NG * PS);
-    rr::put_partials(buf + warp * NG * PS, PS, gq, tq, acc);
+    if (busy) {
+      while (rr::cycles() - met < (uint32_t)p.hold_q) { }
+      uint4 x[NT][KB2], xl[NT][KB2];
+      rr::look(x, q, q_off);
+      if (SPLIT && KB2 == 1) rr::look(xl, q_low, q_off);   // (more blocks: a look that comes too early costs more)
+      if (!rr::await(x, q, q_off, false, p.spin_limit, p.abort_word)) give_up(1, s);
+      __syncwarp();
+      if (SPLIT && KB2 > 1) rr::look(xl, q_low, q_off);
+      float acc[CH2][MT][NT][4];
+      rr::products(acc, w2, x);
+      if (SPLIT) {
+        if (!rr::await(xl, q_low, q_off, false, p.spin_limit, p.abort_word)) give_up(1, s);
+        __syncwarp();
+        rr::add_products(acc, w2, xl);
+      }
+      rr::put_partials(buf + warp * NG * PS, PS, gq, tq, acc);
+    }
     __syncthreads();
     met = rr::cycles();
     const int bad = s_bad[1][s & 1];

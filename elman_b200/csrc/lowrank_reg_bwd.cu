@@ -4,7 +4,7 @@
 namespace elman {
 
 LowRankRegKernel lowrank_reg_bwd_kernel(int kb1, int kb2, int mt, int nt) {
-  return rr::pick_lowrank<true>(kb1, kb2, mt, nt);
+  return rr::pick_lowrank<true, false>(kb1, kb2, mt, nt);
 }
 
 }  // namespace elman

@@ -166,16 +166,8 @@ __device__ __forceinline__ bool await(uint4 (&x)[NT][KB], const char* src, const
 // The products of one warp: acc[mt][nt] += W tile mt (A fragments) times the state's row tile nt
 // over KB blocks of two k-steps.
 template <int CH, int MT, int NT, int KB>
-__device__ __forceinline__ void products(float (&acc)[CH][MT][NT][4], const uint32_t (&w)[MT][KB][8],
-                                         const uint4 (&x)[NT][KB]) {
-#pragma unroll
-  for (int ch = 0; ch < CH; ++ch)
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int u = 0; u < 4; ++u) acc[ch][mt][nt][u] = 0.f;
+__device__ __forceinline__ void add_products(float (&acc)[CH][MT][NT][4], const uint32_t (&w)[MT][KB][8],
+                                             const uint4 (&x)[NT][KB]) {
 #pragma unroll
   for (int kb = 0; kb < KB; ++kb) {
 #pragma unroll
@@ -191,6 +183,20 @@ __device__ __forceinline__ void products(float (&acc)[CH][MT][NT][4], const uint
         mma_bf16(acc[CH - 1][mt][nt], w[mt][kb][4], w[mt][kb][5], w[mt][kb][6], w[mt][kb][7],
                  x[nt][kb].z, x[nt][kb].w);
   }
+}
+
+template <int CH, int MT, int NT, int KB>
+__device__ __forceinline__ void products(float (&acc)[CH][MT][NT][4], const uint32_t (&w)[MT][KB][8],
+                                         const uint4 (&x)[NT][KB]) {
+#pragma unroll
+  for (int ch = 0; ch < CH; ++ch)
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[ch][mt][nt][u] = 0.f;
+  add_products(acc, w, x);
 }
 
 // A warp's accumulators to its part of the partial-sum buffer [NT * 8 rows][stride].
