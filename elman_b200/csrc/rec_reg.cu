@@ -130,11 +130,13 @@ RecRegPlan plan_for(int T, int B, int d, int compact) {
   return pl;
 }
 
-// Options that select a plan of the TMEM kernel select that kernel.
+// Options that select a plan or a part of the TMEM kernel select that kernel (rec_replicas limits the
+// copies of either grid).
 bool rr_enabled() {
   const Options& o = options();
   return o.rec_reg != 1 && o.rec_ksplit == 0 && o.rec_groups == 0 && o.rec_mma_warps == 0 &&
-         o.rec_trace == 0;
+         o.rec_trace == 0 && o.rec_w_tmem == 0 && o.rec_direct_publish == 0 && o.rec_large_batch == 1 &&
+         o.rec_group_cap == 0 && o.rec_fin_groups == 0;
 }
 
 int rr_launch(bool bwd, const RecRegPlan& pl, RecRegParams& p, int* sync, int compact, cudaStream_t stream) {

@@ -58,6 +58,10 @@ int elman_b200_device_status(int* detail, int clear);
  * Tuning and test knobs (process-wide):
  *   "force_generic"  1 = always take the CUDA-core kernels, 0 = default
  *   "spin_limit"     iteration cap of every device-side wait
+ *   "rec_reg"        1 = never the recurrences, and the generation step, that hold their matrices in
+ *                    registers; 0 (default) = wherever they take the shape.  They also leave dense
+ *                    recurrences alone while one of the following options on the
+ *                    tensor-core recurrence (rec_*, but for rec_replicas) is not at its default
  *   "rec_ksplit"     K-split (cluster size) of the tensor-core recurrence, 0 = auto
  *   "rec_groups"     independent batch groups pipelined by the recurrence, 0 = auto
  *   "time_kernels"   1 = bracket the phases of E1/E0 calls with CUDA events
@@ -68,7 +72,7 @@ int elman_b200_device_status(int* detail, int clear);
  *                    recurrence: 0 = auto (forward: each epilogue warp after its own
  *                    stores; backward: a dedicated publisher warp), 1 = epilogue
  *                    warps in both directions, 2 = publisher warp in both.  All
- *                    modes give bit-identical results.
+ *                    modes of that kernel give bit-identical results.
  *   "rec_w_tmem"     where the recurrent weight tile lives: 0 (default) = in tensor memory
  *                    (A operand read from TMEM) where the plan prefers it and it fits, 1 = in
  *                    tensor memory whenever it fits, 2 = always in shared memory; bit-identical
@@ -83,7 +87,7 @@ int elman_b200_device_status(int* detail, int clear);
  *   "rec_large_batch" 1 (default) = batches over 32 rows take the throughput plan of
  *                    the tensor-core recurrence (widest batch group first), 0 = the
  *                    latency plan for every batch size
- *   "rec_replicas"   batch replicas of the tensor-core recurrence's grid for batches over 32:
+ *   "rec_replicas"   batch replicas of a recurrence's grid for larger batches:
  *                    0 (default) = as many copies of the grid as fit on the device, each on
  *                    its own share of the batch (they never wait on each other), 1 = one
  *                    copy, n = at most n.  Results do not depend on it.

@@ -189,7 +189,8 @@ def test_wide_large_batch_forward_shape_of_config4():
 @pytest.mark.parametrize("mode", [1, 2])
 def test_both_publication_modes_give_identical_results(mode):
     inp = orc.make_e1_inputs(20, 32, 512, seed=31)
-    a, _ = run_e1(inp, torch.bfloat16)
+    with option("rec_reg", 1):                  # the kernel with the two modes, at its default
+        a, _ = run_e1(inp, torch.bfloat16)
     with option("rec_direct_publish", mode):
         b, _ = run_e1(inp, torch.bfloat16)
     for k in FWD_BWD_KEYS:
@@ -200,7 +201,8 @@ def test_weights_in_tensor_memory_variant_is_bit_identical():
     """The recurrent weight tile as the MMAs' A operand from tensor memory (1, also the default
     where it fits) or from shared memory (2)."""
     inp = orc.make_e1_inputs(20, 32, 512, seed=32)
-    default, _ = run_e1(inp, torch.bfloat16)
+    with option("rec_reg", 1):
+        default, _ = run_e1(inp, torch.bfloat16)
     with option("rec_w_tmem", 1):
         a, _ = run_e1(inp, torch.bfloat16)
     with option("rec_w_tmem", 2):
@@ -258,16 +260,22 @@ def test_weight_gradients_dual_launch_and_split_k_match_oracle():
         assert orc.rel_err(split[k].float().cpu(), plain[k].float().cpu()) < 5e-3, k
 
 
+@pytest.fixture(params=[1, 0], ids=["tcgen05", "registers"])
+def either_kernel(request):
+    with option("rec_reg", request.param):
+        yield
+
+
 @pytest.mark.parametrize("T,B,d", [(6, 48, 256), (5, 64, 256), (4, 96, 384), (5, 128, 512),
                                    (3, 256, 512), (4, 160, 256), (3, 512, 256)])
-def test_large_batch_plans_match_oracle(T, B, d):
-    """Batches over 32 take the throughput plan (wide batch groups pipelined through the
+def test_large_batch_plans_match_oracle(T, B, d, either_kernel):
+    """Batches over 32 of the tcgen05 kernel take the throughput plan (wide batch groups pipelined through the
     resident weight tile, publisher warp, W in tensor memory when needed): forward and
     backward against the oracle, and against the latency plan."""
     inp = orc.make_e1_inputs(T, B, d, seed=B + d)
     before = _lib.tc_launch_count()
     got, ref = run_e1(inp, torch.bfloat16)
-    assert _lib.tc_launch_count() - before >= 2, "the recurrences must take the tcgen05 kernel"
+    assert _lib.tc_launch_count() - before >= 2, "the recurrences must take a tensor-core kernel"
     assert _lib.device_status()[0] == 0
     assert_close(errors(got, oracle_e1(ref)), TOL[torch.bfloat16], "throughput plan vs oracle")
     with option("rec_large_batch", 0):
@@ -277,7 +285,7 @@ def test_large_batch_plans_match_oracle(T, B, d):
 
 
 @pytest.mark.parametrize("T,B,d", [(5, 128, 512), (4, 256, 256), (3, 192, 384), (6, 256, 2048)])
-def test_batch_replicas_of_the_grid_change_nothing(T, B, d):
+def test_batch_replicas_of_the_grid_change_nothing(T, B, d, either_kernel):
     """Large batches run several independent copies of the recurrence grid, each on its own
     share of the batch groups (option rec_replicas).  Every sequence is computed by the same
     program either way: outputs and data gradients are bit-identical to the single-copy

@@ -58,7 +58,13 @@ def _expect_timeout(kernel_id):
     _lib.device_status(clear=True)
 
 
-def test_recurrence_kernels_give_up_when_a_block_stalls_and_recover():
+@pytest.fixture(params=[0, 1], ids=["registers", "tcgen05"])
+def either_kernel(request):
+    with option("rec_reg", request.param):
+        yield
+
+
+def test_recurrence_kernels_give_up_when_a_block_stalls_and_recover(either_kernel):
     T, B, d = 8, 16, 256
     inp = orc.make_e1_inputs(T, B, d, seed=41)
     dev, ref = round_inputs(inp, torch.bfloat16)
@@ -82,7 +88,7 @@ def test_recurrence_kernels_give_up_when_a_block_stalls_and_recover():
     assert_close(errors(got, oracle_e1(ref)), TOL[torch.bfloat16], "after the give-up")
 
 
-def test_lowrank_kernel_gives_up_when_a_block_withholds_its_share_and_recovers():
+def test_lowrank_kernel_gives_up_when_a_block_withholds_its_share_and_recovers(either_kernel):
     T, B, d, r = 8, 16, 256, 64
     inp = orc.make_e5_inputs(T, B, d, r, seed=42)
     dev, _ = round_inputs(inp, torch.bfloat16)
