@@ -478,6 +478,7 @@ struct SpectralManyParams {
   int* abort_word;
   int* status;
   long spin_limit;
+  int stall_iter;                  // test hook: block 0 never sees its partials of this iteration (-1 off)
   const bf16* W[LT_MAX_LAYERS];
   bf16* u[LT_MAX_LAYERS];
   float* scale[LT_MAX_LAYERS];
@@ -488,15 +489,17 @@ __host__ __device__ inline long spectral_exchange_floats(int d, int NC) {
 }
 
 // Words from other CTAs, when they are there: N at a time, all in flight (at(i) null: none).
+// `stalled` (test hook): never there.
 template <int N, typename At>
-__device__ __forceinline__ void await_words(float (&v)[N], At at, const SpectralManyParams& p, int* bad) {
+__device__ __forceinline__ void await_words(float (&v)[N], At at, const SpectralManyParams& p, int* bad,
+                                            bool stalled = false) {
   uint32_t w[N];
 #pragma unroll
   for (int i = 0; i < N; ++i) w[i] = 0xFFFFFFFFu;
   long spins = 0;
   unsigned long long t_begin = 0;
   while (true) {
-    bool pending = false;
+    bool pending = stalled;
 #pragma unroll
     for (int i = 0; i < N; ++i)
       if (w[i] == 0xFFFFFFFFu) {
@@ -603,7 +606,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) spectral_many_kernel(const __gr
       await_words<NW>(v, [&](int i) -> const float* {
         const int e = e0 + i * SP_THREADS, q = e / rows;
         return e < NC * rows ? ex + ((long)it * NC + q) * d + r0 + e - q * rows : nullptr;
-      }, p, &s_bad);
+      }, p, &s_bad, blockIdx.x == 0 && it == p.stall_iter);
 #pragma unroll
       for (int i = 0; i < NW; ++i) {
         const int e = e0 + i * SP_THREADS, q = e / rows;
@@ -774,7 +777,9 @@ int lm_token(const LmTokenArgs& a, cudaStream_t stream) {
   float* scales = (float*)(ws + act + exb + 256);
   p.status = device_status_ptr();
   p.spin_limit = options().spin_limit;
-  p.stall_layer = (int)options().test_stall_step;
+  const long stall = options().test_stall_step;     // a layer, or 1000 + an iteration of the power iterations
+  p.stall_layer = stall < 1000 ? (int)stall : -1;
+  q.stall_iter = stall < 1000 ? -1 : (int)(stall - 1000);
   // read 16 bytes at a time; in feature pairs
   uintptr_t wide = (uintptr_t)a.embedding | (uintptr_t)a.norm | (uintptr_t)a.head | (uintptr_t)ws;
   uintptr_t narrow = 0;

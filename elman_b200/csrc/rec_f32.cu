@@ -39,6 +39,7 @@ struct RecF32Params {
   int* status;
   long spin_limit;
   int self_gate;
+  int stall_step;         // test hook: block 0 never sees its input of this step (-1 off)
 };
 
 template <bool BWD, int KW>
@@ -106,6 +107,7 @@ __global__ void __launch_bounds__(RR_THREADS, 1) rec_f32_kernel(const RecF32Para
 #pragma unroll
   for (int s = 0; s < RR_AHEAD - 1; ++s) fetch(s, at + s * step_bytes);
   float db_acc = 0.f;
+  const int stall_step = blockIdx.x == 0 ? p.stall_step : -1;
   __syncthreads();
 
   for (int s = 0; s < T; ++s, at += step_bytes) {
@@ -140,7 +142,7 @@ __global__ void __launch_bounds__(RR_THREADS, 1) rec_f32_kernel(const RecF32Para
 #pragma unroll
     for (int j = 0; j < LOOKS; ++j) x[j] = rr::ld_relaxed_v4(src + x_off[0][j]);
     while (s > 0) {
-      uint32_t top = 0;
+      uint32_t top = s == stall_step ? 0xFFFFFFFFu : 0u;
 #pragma unroll
       for (int j = 0; j < LOOKS; ++j) top = max(top, x_on[j] ? rr::largest(x[j]) : 0u);
       if (top != 0xFFFFFFFFu) break;
@@ -243,6 +245,7 @@ int f32_launch(bool bwd, RecF32Params& p, int* sync, cudaStream_t stream) {
   p.abort_word = sync;
   p.status = device_status_ptr();
   p.spin_limit = options().spin_limit;
+  p.stall_step = (int)options().test_stall_step;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((per < groups ? per : groups) * p.cpg);
   cfg.blockDim = dim3(RR_THREADS);

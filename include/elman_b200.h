@@ -97,7 +97,8 @@ int elman_b200_device_status(int* detail, int clear);
  *                    on it together, for launches whose blocks wait for one another
  *   "test_stall_step" failure-detection test hook, -1 (default) = off.  With a value k >= 1
  *                    thread block 0 of the next tensor-core launches (recurrences: at time
- *                    step k; projection GEMMs: at K iteration k) waits for something that
+ *                    step k; projection GEMMs: at K iteration k; generation step: at layer k, or
+ *                    for 1000 + i at iteration i of its power iterations) waits for something that
  *                    nothing delivers.  The wait runs out after "spin_limit" polls, the
  *                    kernel records ELMAN_ERR_TIMEOUT in the status word, every block gives
  *                    up and the launch returns; its results are invalid.  Nothing faults.

@@ -5,7 +5,7 @@ for a product against fp64 (a sum of K terms is off by about sqrt(K) 2^-24, 2.4e
 import pytest
 import torch
 
-from _gpu_cases import TOL, assert_close, errors, option, oracle_e1, run_e1
+from _gpu_cases import TOL, assert_close, errors, option, oracle_e1, round_inputs, run_e1
 from elman_b200 import _lib
 from elman_b200 import hasty_pytorch_lib as H
 from oracle import elman_oracle as orc
@@ -39,3 +39,19 @@ def test_products_of_every_form(op, M, N, K):
     assert orc.rel_err(out.double().cpu(), base) < 1e-6
     out = H.gemm(op, A.cuda(), B.cuda(), out=out, accumulate=True)
     assert orc.rel_err(out.double().cpu(), base + want) < 1e-6
+
+
+def test_recurrence_gives_up_when_a_block_stalls_and_recovers():
+    inp = orc.make_e1_inputs(8, 6, 260, seed=9)
+    dev, ref = round_inputs(inp, torch.float32)
+    good, _ = run_e1(inp, torch.float32)
+    _lib.device_status(clear=True)
+    for call in (lambda: H.e1_recurrence_forward(True, dev["x"], dev["z"], dev["h0"], dev["W_h"]),
+                 lambda: H.e1_recurrence_backward(dev["W_h"], dev["z"], good["h"], good["v"], dev["d_output"])):
+        with option("spin_limit", 5000), option("test_stall_step", 4):
+            call()
+            torch.cuda.synchronize()
+        code, detail = _lib.device_status(clear=True)
+        assert code == 3 and detail >> 24 == 1 and detail & 0xFFFFFF in (4, 5)   # the block, or one behind it
+    got, _ = run_e1(inp, torch.float32)
+    assert_close(errors(got, oracle_e1(ref)), TOL[torch.float32], "after the give-up")

@@ -65,17 +65,27 @@ def test_changed_parameters_are_seen_and_a_token_outside_the_vocabulary_is_repor
     assert code == 3 and detail >> 24 == 8
 
 
-def test_gives_up_when_a_block_stalls_and_recovers():
-    model = _model(64, 3, "none")
+@pytest.mark.parametrize("mode,stall", [("none", 1), ("spectral_norm", 1), ("spectral_norm", 1000),
+                                        ("spectral_norm", 1002)])
+def test_gives_up_when_a_block_stalls_and_recovers(mode, stall):
+    """A layer's input, and a round of the power iterations in front of it (1000 + its number)."""
+    model = _model(64, 3, mode)
     tok = torch.tensor([[3], [5]]).cuda()
+    us = [torch.full((64,), 0.125, dtype=torch.bfloat16, device="cuda") for _ in range(3)]
+
+    def step():
+        for layer, u in zip(model.layers, us):
+            layer.cell._spectral_u = u.clone()
+        return model(tok)
+
     with torch.no_grad():
-        want = model(tok)
-        with option("spin_limit", 5000), option("test_stall_step", 1):
-            model(tok)
+        want = step()
+        with option("spin_limit", 5000), option("test_stall_step", stall):
+            step()
         torch.cuda.synchronize()
         code, detail = _lib.device_status(clear=True)
         assert code == 3 and detail >> 24 == 8
-        assert torch.equal(model(tok), want)
+        assert torch.equal(step(), want)
 
 
 def test_bias_between_two_words_goes_layer_by_layer():
