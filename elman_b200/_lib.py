@@ -38,6 +38,7 @@ SIGNATURES = {
     "elman_b200_recurrence_trace": (_I, [_c.POINTER(_c.c_longlong), _I]),
     "elman_b200_launch_count": (_L, []),
     "elman_b200_tc_launch_count": (_L, []),
+    "elman_b200_recurrence_launch_count": (_L, [_c.c_char_p]),
     "elman_e1_forward_workspace": (_Z, [_I, _I, _I, _I]),
     "elman_e1_forward": (_I, [_I, _I, _I, _I, _I] + [_P] * 6 + [_P] * 3 + [_P, _Z, _P]),
     "elman_e1_forward_static_scratch_bytes": (_Z, []),
@@ -160,6 +161,10 @@ def launch_count() -> int:
 
 def tc_launch_count() -> int:
     return int(load().elman_b200_tc_launch_count())
+
+
+def recurrence_launch_count(kernel: str) -> int:
+    return int(load().elman_b200_recurrence_launch_count(kernel.encode()))
 
 
 def last_timing_ms(phase: int) -> float:

@@ -32,8 +32,10 @@ Options& options() {
 
 static std::atomic<long> g_launches{0};
 static std::atomic<long> g_tc_launches{0};
-void count_launch(bool tensor_core) {
+static std::atomic<long> g_rec_launches[REC_KERNELS];
+void count_launch(bool tensor_core, RecKernel kernel) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
+  g_rec_launches[kernel].fetch_add(1, std::memory_order_relaxed);
   if (tensor_core) g_tc_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
@@ -402,6 +404,14 @@ int elman_b200_recurrence_trace(long long* dst, int max_entries) {
 
 long elman_b200_launch_count(void) { return g_launches.load(); }
 long elman_b200_tc_launch_count(void) { return g_tc_launches.load(); }
+
+long elman_b200_recurrence_launch_count(const char* kernel) {
+  static const char* const names[REC_KERNELS] = {"other", "rec_reg", "rec_turns", "rec_f32", "rec_tc", "rec_simt",
+                                                 "lowrank_reg", "lowrank_tc"};
+  for (int i = 0; i < REC_KERNELS; ++i)
+    if (kernel != nullptr && !strcmp(kernel, names[i])) return g_rec_launches[i].load();
+  return -1;
+}
 
 int elman_b200_recurrence_blocks(int dtype, int flags, int T, int B, int d) {
   if (T <= 0 || B <= 0 || d <= 0) return 0;

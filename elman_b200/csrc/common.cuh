@@ -64,7 +64,10 @@ struct Options {
   long test_stall_step = -1;
 };
 Options& options();
-void count_launch(bool tensor_core);
+// `kernel`: for the kernels that carry a recurrence, so that a test can tell which of them ran.
+enum RecKernel { REC_KERNEL_OTHER, REC_KERNEL_REG, REC_KERNEL_TURNS, REC_KERNEL_F32, REC_KERNEL_TC, REC_KERNEL_SIMT,
+                 REC_KERNEL_LOWRANK_REG, REC_KERNEL_LOWRANK_TC, REC_KERNELS };
+void count_launch(bool tensor_core, RecKernel kernel = REC_KERNEL_OTHER);
 
 // Host-visible status word of the current device (mapped pinned memory).
 // Device code writes a non-zero code there when a bounded wait gives up.

@@ -118,7 +118,7 @@ int lowrank_reg(const LowRankRegArgs& a, cudaStream_t stream) {
     const int groups = (p.b_hi - b + 8 * pl.nt - 1) / (8 * pl.nt);
     cfg.gridDim = dim3(groups * pl.cpg);
     ELMAN_RETURN_IF(launch_together(kern, cfg, p));
-    count_launch(true);
+    count_launch(true, REC_KERNEL_LOWRANK_REG);
   }
   const int rows = (a.B + 8 * pl.nt - 1) / (8 * pl.nt);
   if (bwd && rows > 1) return fold_db_rows(a.db, a.d, rows, stream);

@@ -651,7 +651,7 @@ int lowrank_tc(const LowRankTcArgs& a, cudaStream_t stream) {
     ELMAN_CUDA_CHECK(cudaLaunchKernelEx(&cfg, lowrank_tc_kernel<false>, tmU, tmState, tmIn[0],
                                         tmIn[1], tmIn[2], tmIn[3], tmOut[0], tmOut[1], has_out0, p));
   }
-  count_launch(true);
+  count_launch(true, REC_KERNEL_LOWRANK_TC);
   return ELMAN_OK;
 }
 

@@ -265,7 +265,7 @@ int f32_launch(bool bwd, RecF32Params& p, int* sync, cudaStream_t stream) {
     p.b_hi = (g + per) * F32_NG < p.B ? (g + per) * F32_NG : p.B;
     cfg.gridDim = dim3((p.b_hi - p.b_lo + F32_NG - 1) / F32_NG * p.cpg);
     ELMAN_RETURN_IF(launch_together(kern, cfg, p));
-    count_launch(false);
+    count_launch(false, REC_KERNEL_F32);
   }
   if (bwd && groups > 1) return fold_db_rows(p.db, p.d, groups, stream);
   return ELMAN_OK;

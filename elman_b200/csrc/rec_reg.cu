@@ -181,7 +181,7 @@ int rr_launch(bool bwd, const RecRegPlan& pl, RecRegParams& p, int* sync, int co
   const size_t slot = (size_t)p.B * p.d * sizeof(bf16);
   ELMAN_CUDA_CHECK(cudaMemsetAsync((char*)p.state + (bwd ? 0 : slot), 0xFF, (size_t)p.T * slot, stream));
   ELMAN_RETURN_IF(launch_together(kern, cfg, p));
-  count_launch(true);
+  count_launch(true, turns ? REC_KERNEL_TURNS : REC_KERNEL_REG);
   return ELMAN_OK;
 }
 

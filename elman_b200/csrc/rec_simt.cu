@@ -414,7 +414,7 @@ int launch_coop(Kern kern, P& params, int grid, size_t smem, cudaStream_t stream
   void* args[] = {&params};
   ELMAN_CUDA_CHECK(cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(NTHREADS), args,
                                                smem, stream));
-  count_launch(false);
+  count_launch(false, REC_KERNEL_SIMT);
   return ELMAN_OK;
 }
 

@@ -1118,7 +1118,7 @@ int launch_rec_tc_fg(const RecPlan& pl, RecTcParams& p, const void* W, const voi
     return set_error(ELMAN_ERR_UNSUPPORTED, "recurrence grid of %d CTAs is not co-resident (%d clusters of %d fit)",
                      (int)cfg.gridDim.x, max_clusters, pl.S);
   ELMAN_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tmW, tmState, tmI[0], tmI[1], tmI[2], tmI[3], p));
-  count_launch(true);
+  count_launch(true, REC_KERNEL_TC);
   return ELMAN_OK;
 }
 

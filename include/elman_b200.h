@@ -147,6 +147,9 @@ int elman_b200_recurrence_trace(long long* dst, int max_entries);
 long elman_b200_launch_count(void);
 /* Of those, launches that took a tcgen05 tensor-core kernel. */
 long elman_b200_tc_launch_count(void);
+/* Launches of one of the kernels that carry a recurrence: "rec_reg", "rec_turns", "rec_f32", "rec_tc",
+ * "rec_simt" (dense and low-rank), "lowrank_reg", "lowrank_tc"; -1 for another name. */
+long elman_b200_recurrence_launch_count(const char* kernel);
 
 /* ---------------------------------------------------------------------------
  * E1 — gated Elman cell.

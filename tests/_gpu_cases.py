@@ -23,6 +23,15 @@ def option(name, value):
         _lib.set_option(name, old)
 
 
+@contextlib.contextmanager
+def launches_of(kernel, n):
+    """Exactly n launches of this recurrence kernel inside."""
+    before = _lib.recurrence_launch_count(kernel)
+    yield
+    ran = _lib.recurrence_launch_count(kernel) - before
+    assert ran == n, f"{ran} launches of {kernel}, not {n}"
+
+
 def round_inputs(inp, dtype):
     """Round every input to `dtype` first; the oracle gets the rounded values in fp32."""
     dev = {k: v.to(dtype).cuda().contiguous() for k, v in inp.items()}

@@ -5,7 +5,7 @@ for a product against fp64 (a sum of K terms is off by about sqrt(K) 2^-24, 2.4e
 import pytest
 import torch
 
-from _gpu_cases import TOL, assert_close, errors, option, oracle_e1, round_inputs, run_e1
+from _gpu_cases import TOL, assert_close, errors, launches_of, option, oracle_e1, round_inputs, run_e1
 from elman_b200 import _lib
 from elman_b200 import hasty_pytorch_lib as H
 from oracle import elman_oracle as orc
@@ -13,11 +13,12 @@ from oracle import elman_oracle as orc
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("T,B,d", [(1, 1, 8), (7, 5, 12), (5, 4, 184), (6, 17, 260), (4, 3, 516),
-                                   (3, 33, 1000), (3, 2, 1024)])
-def test_recurrence_matches_oracle(T, B, d):
+@pytest.mark.parametrize("T,B,d,slices", [(1, 1, 8, 1), (7, 5, 12, 1), (5, 4, 184, 1), (6, 17, 260, 1), (4, 3, 516, 1),
+                                          (3, 33, 1000, 3), (3, 2, 1024, 1)])
+def test_recurrence_matches_oracle(T, B, d, slices):
     inp = orc.make_e1_inputs(T, B, d, seed=d + B)
-    got, ref = run_e1(inp, torch.float32)
+    with launches_of("rec_f32", 2 * slices):
+        got, ref = run_e1(inp, torch.float32)
     assert _lib.device_status()[0] == 0
     assert_close(errors(got, oracle_e1(ref)), TOL[torch.float32], f"fp32 T{T} B{B} d{d}")
     with option("rec_reg", 1):      # the cooperative kernel: the same arithmetic in another order

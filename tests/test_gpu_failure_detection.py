@@ -41,7 +41,7 @@ def test_wait_probe_times_out_and_context_survives():
 # entry point must refuse, and after clearing the same call must match the oracle.
 # ---------------------------------------------------------------------------
 from oracle import elman_oracle as orc  # noqa: E402
-from tests._gpu_cases import TOL, assert_close, errors, option, oracle_e1, oracle_e5  # noqa: E402
+from tests._gpu_cases import TOL, assert_close, errors, launches_of, option, oracle_e1, oracle_e5  # noqa: E402
 from tests._gpu_cases import round_inputs, run_e1, run_e5  # noqa: E402
 
 KID_REC_TC_FWD, KID_REC_TC_BWD, KID_GEMM_TC, KID_LOWRANK_TC = 2, 3, 4, 7
@@ -61,7 +61,7 @@ def _expect_timeout(kernel_id):
 @pytest.fixture(params=[0, 1], ids=["registers", "tcgen05"])
 def either_kernel(request):
     with option("rec_reg", request.param):
-        yield
+        yield ("rec_tc", "lowrank_tc") if request.param else ("rec_reg", "lowrank_reg")
 
 
 def test_recurrence_kernels_give_up_when_a_block_stalls_and_recover(either_kernel):
@@ -69,16 +69,14 @@ def test_recurrence_kernels_give_up_when_a_block_stalls_and_recover(either_kerne
     inp = orc.make_e1_inputs(T, B, d, seed=41)
     dev, ref = round_inputs(inp, torch.bfloat16)
     _lib.device_status(clear=True)
-    before = _lib.tc_launch_count()
-    with option("spin_limit", 5000), option("test_stall_step", 5):
+    with option("spin_limit", 5000), option("test_stall_step", 5), launches_of(either_kernel[0], 1):
         H.mamba_gated_elman_forward(True, dev["x"], dev["z"], dev["h0"], dev["W_x"], dev["W_h"],
                                     dev["b"])
         _expect_timeout(KID_REC_TC_FWD)
-    assert _lib.tc_launch_count() > before
     # a clean forward gives the states the backward needs; then stall the backward kernel
     h, out, v = H.mamba_gated_elman_forward(True, dev["x"], dev["z"], dev["h0"], dev["W_x"],
                                             dev["W_h"], dev["b"])
-    with option("spin_limit", 5000), option("test_stall_step", 5):
+    with option("spin_limit", 5000), option("test_stall_step", 5), launches_of(either_kernel[0], 1):
         H.mamba_gated_elman_backward(dev["W_x"], dev["W_h"], dev["x"], dev["z"], h, v,
                                      dev["d_output"])
         _expect_timeout(KID_REC_TC_BWD)
@@ -94,7 +92,7 @@ def test_lowrank_kernel_gives_up_when_a_block_withholds_its_share_and_recovers(e
     dev, _ = round_inputs(inp, torch.bfloat16)
     w = [dev[k] for k in ("U_h", "V_h", "U_x", "V_x", "U_z", "V_z")]
     _lib.device_status(clear=True)
-    with option("spin_limit", 5000), option("test_stall_step", 5):
+    with option("spin_limit", 5000), option("test_stall_step", 5), launches_of(either_kernel[1], 1):
         H.pure_lowrank_elman_forward(True, dev["x"], dev["h0"], *w, dev["b"])
         _expect_timeout(KID_LOWRANK_TC)
     got, ref = run_e5(inp, torch.bfloat16)

@@ -5,7 +5,7 @@ tolerance of the other parity tests."""
 import pytest
 import torch
 
-from _gpu_cases import TOL, assert_close, errors, option, oracle_e1, run_e1
+from _gpu_cases import TOL, assert_close, errors, launches_of, option, oracle_e1, run_e1
 from elman_b200 import _lib
 from elman_b200 import hasty_pytorch_lib as H
 from oracle import elman_oracle as orc
@@ -18,9 +18,8 @@ pytestmark = pytest.mark.gpu
                                    (3, 61, 1000), (3, 5, 2040), (3, 64, 1536)])
 def test_ragged_shapes_match_oracle(T, B, d):
     inp = orc.make_e1_inputs(T, B, d, seed=7 * d + B)
-    before = _lib.tc_launch_count()
-    got, ref = run_e1(inp, torch.bfloat16)
-    assert _lib.tc_launch_count() - before >= 2, "both recurrences must take the kernel"
+    with launches_of("rec_reg", 2):
+        got, ref = run_e1(inp, torch.bfloat16)
     assert _lib.device_status()[0] == 0
     assert_close(errors(got, oracle_e1(ref)), TOL[torch.bfloat16], f"T{T} B{B} d{d}")
 
@@ -57,22 +56,21 @@ def test_contexts_with_too_little_room_take_another_kernel():
     lm = LadderLM(vocab_size=64, dim=64, depth=2, level=1).cuda().bfloat16().eval()
     tok = torch.tensor([[3]]).cuda()
     for limit in (0, 1):
+        own = 2 if limit == 0 else 0
         with option("test_resident_blocks", limit):
-            before = _lib.tc_launch_count()
-            got, ref = run_e1(inp, torch.bfloat16)
-            tc = _lib.tc_launch_count() - before
+            with launches_of("rec_reg", own):
+                got, ref = run_e1(inp, torch.bfloat16)
             assert_close(errors(got, oracle_e1(ref)), TOL[torch.bfloat16], f"bf16, limit {limit}")
-            got, ref = run_e1(inp, torch.float32)
+            with launches_of("rec_f32", own):
+                got, ref = run_e1(inp, torch.float32)
             assert_close(errors(got, oracle_e1(ref)), TOL[torch.float32], f"fp32, limit {limit}")
-            got, ref = run_e5(low, torch.bfloat16)
+            with launches_of("lowrank_reg", own):
+                got, ref = run_e5(low, torch.bfloat16)
             assert_close(errors(got, oracle_e5(ref)), TOL[torch.bfloat16], f"low rank, limit {limit}")
             before = _lib.launch_count()
             with torch.no_grad():
                 lm(tok)
             assert (_lib.launch_count() - before > 2) == (limit == 1)
-        if limit == 0:
-            free = tc
-    assert tc == free - 2, "both recurrences should have left the register kernel"
     assert _lib.device_status()[0] == 0
 
 

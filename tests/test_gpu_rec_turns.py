@@ -6,7 +6,7 @@ with the bf16 tolerance of the other parity tests."""
 import pytest
 import torch
 
-from _gpu_cases import TOL, assert_close, errors, option, oracle_e1, round_inputs
+from _gpu_cases import TOL, assert_close, errors, launches_of, option, oracle_e1, round_inputs
 from elman_b200 import _lib
 from elman_b200 import hasty_pytorch_lib as H
 from oracle import elman_oracle as orc
@@ -25,25 +25,29 @@ def run_compact(inp, flags=H.FLAG_COMPACT):
 
 
 @pytest.mark.parametrize("T,B,d", [(5, 9, 1280), (4, 33, 952), (5, 64, 520), (3, 61, 1000), (3, 17, 2040),
-                                   (4, 20, 1536), (3, 40, 1792), (6, 48, 264), (5, 40, 768), (6, 20, 768),
+                                   (4, 20, 1536), (3, 24, 1800), (6, 48, 264), (5, 40, 768), (6, 20, 768),
                                    (1, 24, 1280)])
 def test_ragged_shapes_match_oracle(T, B, d):
     inp = orc.make_e1_inputs(T, B, d, seed=5 * d + B)
     blocks = H.recurrence_blocks(torch.bfloat16, T, B, d, H.FLAG_COMPACT)
     assert 0 < blocks <= H.recurrence_blocks(torch.bfloat16, T, B, d)
     assert blocks < (B + 7) // 8 * ((d + 63) // 64), "several groups on one set of CTAs"
-    got, ref = run_compact(inp)
+    with launches_of("rec_turns", 2):
+        got, ref = run_compact(inp)
     assert _lib.device_status()[0] == 0
     assert_close(errors(got, oracle_e1(ref)), TOL[torch.bfloat16], f"T{T} B{B} d{d}")
 
 
-@pytest.mark.parametrize("T,B,d", [(4, 65, 64), (3, 130, 520), (3, 100, 952), (2, 250, 1280), (2, 90, 2048),
-                                   (3, 64, 1792)])
-def test_large_batches_match_oracle(T, B, d):
-    """Without the flag: more groups than the device has CTAs for; E1, E1 without a backward pass,
-    and the state as its own gate (E33)."""
+@pytest.mark.parametrize("T,B,d,kernel", [(4, 65, 64, "rec_reg"), (3, 130, 520, "rec_turns"), (3, 100, 952, "rec_turns"),
+                                          (2, 250, 1280, "rec_turns"), (2, 90, 2048, "rec_turns"),
+                                          (3, 64, 1792, "rec_turns"), (2, 1024, 384, "rec_turns")])
+def test_large_batches_match_oracle(T, B, d, kernel):
+    """Without the flag: more groups than the device has CTAs for (the first case: a CTA for each, but more
+    than the 64 rows the plans of rec_reg go up to); E1, E1 without a backward pass, and the state as its
+    own gate (E33)."""
     inp = orc.make_e1_inputs(T, B, d, seed=d - B)
-    got, ref = run_compact(inp, 0)
+    with launches_of(kernel, 2):
+        got, ref = run_compact(inp, 0)
     assert _lib.device_status()[0] == 0
     assert_close(errors(got, oracle_e1(ref)), TOL[torch.bfloat16], f"T{T} B{B} d{d}")
     dev, _ = round_inputs(inp, torch.bfloat16)
@@ -56,6 +60,16 @@ def test_large_batches_match_oracle(T, B, d):
     g = orc.e33_backward(ref["W_x"], ref["W_h"], ref["x"], f["h"], f["v"], ref["d_output"])
     assert_close(errors(dict(h=h, output=out, v=v, dx=dx, dW_x=dWx, dW_h=dWh, db=db), {**f, **g}),
                  TOL[torch.bfloat16], "self gate")
+
+
+@pytest.mark.parametrize("T,B,d", [(2, 576, 256), (2, 640, 1280), (3, 256, 2048)])
+def test_larger_batches_stay_with_the_tcgen05_kernel(T, B, d):
+    """Over 512 rows, or six turns of 32 rows of W."""
+    inp = orc.make_e1_inputs(T, B, d, seed=B)
+    with launches_of("rec_tc", 2):
+        got, ref = run_compact(inp, 0)
+    assert _lib.device_status()[0] == 0
+    assert_close(errors(got, oracle_e1(ref)), TOL[torch.bfloat16], f"T{T} B{B} d{d}")
 
 
 def test_long_chain_agrees_with_one_group_per_set():
