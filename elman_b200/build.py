@@ -2,7 +2,6 @@
 
     python -m elman_b200.build            # build if sources are newer than the .so
     python -m elman_b200.build --force
-    python -m elman_b200.build --microbench   # also the standalone program under csrc/microbench
 
 The result, elman_b200/lib/libelman_b200.so, is a plain C-ABI shared library
 (see include/elman_b200.h); it does not link against PyTorch.
@@ -81,20 +80,5 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
-def build_microbench() -> str:
-    """The standalone measurement program under csrc/microbench (MMA issue rate, cluster exchange)."""
-    src = os.path.join(CSRC, "microbench", "mma_issue_and_cluster_exchange.cu")
-    exe = os.path.join(LIBDIR, "mma_issue_and_cluster_exchange")
-    if os.path.exists(exe) and os.path.getmtime(exe) >= max(
-            os.path.getmtime(src), os.path.getmtime(os.path.join(CSRC, "sm100_ptx.cuh"))):
-        return exe
-    os.makedirs(LIBDIR, exist_ok=True)
-    subprocess.check_call([find_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3",
-                           "-std=c++17", "-lineinfo", "-o", exe, src])
-    return exe
-
-
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="-v" in sys.argv))
-    if "--microbench" in sys.argv:
-        print(build_microbench())
