@@ -107,6 +107,13 @@ inline size_t lt_smem(int d, int nt) {
          (size_t)2 * RR_WARPS * 8 * nt * LT_PS * sizeof(float);
 }
 
+// Waits for the copies that were last sent for, by group.  A call: inlined, the path that no launch should
+// take costs the kernel 36 more bytes of spills and 2 % of its time at 27 sequences.
+__device__ __noinline__ void land(uint64_t* landed, const int* sent) {
+  int none = 0;
+  if (threadIdx.x < 3) ptx::mbar_wait(&landed[threadIdx.x], (uint32_t)sent[threadIdx.x] & 1u, 1L << 40, &none);
+}
+
 template <int KB, int NT, int TURNS>
 __global__ void __launch_bounds__(LT_THREADS, 1) lm_token_kernel(const __grid_constant__ LmTokenParams p) {
   constexpr int ROWS = 8 * NT;              // sequences of a turn
@@ -427,10 +434,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) lm_token_kernel(const __grid_co
     // own memory and always arrive; the wait's time limit is its bound.
     settle_norm();
     __syncthreads();
-    if (tid < 3) {
-      int none = 0;
-      ptx::mbar_wait(&landed[tid], (uint32_t)s_sent[tid] & 1u, 1L << 40, &none);
-    }
+    land(landed, s_sent);
     __syncthreads();
     return;
   }
@@ -478,7 +482,7 @@ struct SpectralManyParams {
   int* abort_word;
   int* status;
   long spin_limit;
-  int stall_iter;                  // test hook: block 0 never sees its partials of this iteration (-1 off)
+  int stall_iter;                  // test hook: block 0 waits in this iteration for what never comes (-1 off)
   const bf16* W[LT_MAX_LAYERS];
   bf16* u[LT_MAX_LAYERS];
   float* scale[LT_MAX_LAYERS];
@@ -489,17 +493,15 @@ __host__ __device__ inline long spectral_exchange_floats(int d, int NC) {
 }
 
 // Words from other CTAs, when they are there: N at a time, all in flight (at(i) null: none).
-// `stalled` (test hook): never there.
 template <int N, typename At>
-__device__ __forceinline__ void await_words(float (&v)[N], At at, const SpectralManyParams& p, int* bad,
-                                            bool stalled = false) {
+__device__ __forceinline__ void await_words(float (&v)[N], At at, const SpectralManyParams& p, int* bad) {
   uint32_t w[N];
 #pragma unroll
   for (int i = 0; i < N; ++i) w[i] = 0xFFFFFFFFu;
   long spins = 0;
   unsigned long long t_begin = 0;
   while (true) {
-    bool pending = stalled;
+    bool pending = false;
 #pragma unroll
     for (int i = 0; i < N; ++i)
       if (w[i] == 0xFFFFFFFFu) {
@@ -526,6 +528,8 @@ __device__ __forceinline__ void await_words(float (&v)[N], At at, const Spectral
   for (int i = 0; i < N; ++i) v[i] = __uint_as_float(w[i]);
 }
 
+// STALL: with the test hook (its one comparison cost 0.6 of 25 us).
+template <bool STALL>
 __global__ void __launch_bounds__(SP_THREADS, 1) spectral_many_kernel(const __grid_constant__ SpectralManyParams p) {
   extern __shared__ __align__(16) float sp_smem[];
   __shared__ float s_red[SP_THREADS / 32];
@@ -600,13 +604,17 @@ __global__ void __launch_bounds__(SP_THREADS, 1) spectral_many_kernel(const __gr
       rr::st_relaxed_u32(mine + col, __float_as_uint(v));
     }
     // ---- my columns: everybody's partials, and the norm of the u they came from ----
+    if (STALL && it == p.stall_iter && blockIdx.x == 0 && tid == 0) {   // (no square sums come before iteration 1)
+      float v[1];
+      await_words<1>(v, [&](int) { return ex_sq; }, p, &s_bad);
+    }
     constexpr int NW = 4;
     for (int e0 = tid; e0 < NC * rows; e0 += NW * SP_THREADS) {
       float v[NW];
       await_words<NW>(v, [&](int i) -> const float* {
         const int e = e0 + i * SP_THREADS, q = e / rows;
         return e < NC * rows ? ex + ((long)it * NC + q) * d + r0 + e - q * rows : nullptr;
-      }, p, &s_bad, blockIdx.x == 0 && it == p.stall_iter);
+      }, p, &s_bad);
 #pragma unroll
       for (int i = 0; i < NW; ++i) {
         const int e = e0 + i * SP_THREADS, q = e / rows;
@@ -818,12 +826,13 @@ int lm_token(const LmTokenArgs& a, cudaStream_t stream) {
   sp_cfg.gridDim = dim3((n_normed < sp.per_launch ? n_normed : sp.per_launch) * sp.NC);
   sp_cfg.blockDim = dim3(SP_THREADS);
   sp_cfg.dynamicSmemBytes = sp.smem;
+  void (*const power)(const SpectralManyParams) = q.stall_iter < 0 ? spectral_many_kernel<false> : spectral_many_kernel<true>;
   ELMAN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_SMEM_LIMIT));
   if (!fits_together((const void*)kern, cfg)) return ELMAN_ERR_UNSUPPORTED;
   if (n_normed > 0) {
-    ELMAN_CUDA_CHECK(cudaFuncSetAttribute(spectral_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    ELMAN_CUDA_CHECK(cudaFuncSetAttribute(power, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           SP_SMEM_LIMIT));
-    if (!fits_together((const void*)spectral_many_kernel, sp_cfg)) return ELMAN_ERR_UNSUPPORTED;
+    if (!fits_together((const void*)power, sp_cfg)) return ELMAN_ERR_UNSUPPORTED;
   }
   ELMAN_CUDA_CHECK(cudaMemsetAsync(ws, 0xFF, act + exb + 256, stream));
   for (int i = 0; i < n_normed; i += sp.per_launch) {
@@ -834,7 +843,7 @@ int lm_token(const LmTokenArgs& a, cudaStream_t stream) {
     }
     q.exchange = (float*)(ws + act) + (size_t)i * ex_floats;
     sp_cfg.gridDim = dim3(m * sp.NC);
-    const int rc = launch_together(spectral_many_kernel, sp_cfg, q);
+    const int rc = launch_together(power, sp_cfg, q);
     if (rc != ELMAN_OK) return i == 0 ? rc : too_late(rc);
     count_launch(false);
   }
