@@ -37,9 +37,10 @@ METRIC = "E1 layer fwd+bwd tokens/s @ d1280 B32 T512"
 UNIT = "tokens/s"
 T, B, D = 512, 32, 1280
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
-# DRAM bytes per launch of the dominant kernel from the committed ncu capture
-# (profiles/), or None while no capture of the current kernel exists.
-NCU_TRAFFIC_BYTES = {"rec_tc_kernel<fwd>": 170.1e6, "rec_tc_kernel<bwd>": 231.1e6}  # profiles/rec_tc_kernel_e1_c1.md
+# DRAM bytes per launch of a recurrence kernel at this workload, from ncu captures (dram__bytes_read.sum +
+# dram__bytes_write.sum); None for a kernel without one.
+NCU_TRAFFIC_BYTES = {"rec_reg_kernel<fwd>": 167.7e6, "rec_reg_kernel<bwd>": 227.4e6,
+                     "rec_tc_kernel<fwd>": 170.1e6, "rec_tc_kernel<bwd>": 231.1e6}
 
 
 def host_topology():
@@ -703,11 +704,13 @@ def main():
 
     _lib.set_option("time_kernels", 1)
     launches0, tc0 = _lib.launch_count(), _lib.tc_launch_count()
+    rec0 = {k: _lib.recurrence_launch_count(k) for k in ("rec_reg", "rec_turns", "rec_tc", "rec_simt")}
     sampler.begin()
     total_ms, wall, phase_ms = timed(step_device, args.steps, phases=True)
     sampler.end()
     launches = _lib.launch_count() - launches0
     tc_launches = _lib.tc_launch_count() - tc0
+    rec_kernel = max(rec0, key=lambda k: _lib.recurrence_launch_count(k) - rec0[k])
     _lib.set_option("time_kernels", 0)
 
     for _ in range(3):
@@ -789,10 +792,10 @@ def main():
         achieved_tf = rec_flops / (dom_ms / 1e3) / 1e12 if dom_ms > 0 else 0.0
         peak_tf = float(peaks.get("bf16_tflops", FALLBACK_PEAKS["bf16_tflops"]))
         roofline = {
-            "kernel": f"rec_tc_kernel<{dom}>", "bound": "tensor",
+            "kernel": f"{rec_kernel}_kernel<{dom}>", "bound": "tensor",
             "achieved": achieved_tf, "peak": peak_tf, "unit": "TFLOP/s",
             "frac": achieved_tf / peak_tf if peak_tf else None,
-            "traffic": NCU_TRAFFIC_BYTES.get(f"rec_tc_kernel<{dom}>"),
+            "traffic": NCU_TRAFFIC_BYTES.get(f"{rec_kernel}_kernel<{dom}>"),
             "peak_source": f"{peaks_kind} (bf16_tflops burst; sustained "
                            f"{peaks.get('bf16_tflops_sustained')})",
             "note": "per-step recurrence at B=32 is latency-bound (grid-wide dependency every "
