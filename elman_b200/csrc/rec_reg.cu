@@ -1,6 +1,8 @@
 // Plans and launches of the register-resident recurrence (rec_reg.cuh).
 #include <limits.h>
 
+#include <atomic>
+
 #include "rec_reg_table.cuh"
 
 namespace elman {
@@ -188,13 +190,18 @@ int rr_launch(bool bwd, const RecRegPlan& pl, RecRegParams& p, int* sync, int co
 }  // namespace
 
 int rec_reg_sms() {
-  static int sms[64] = {0};
-  int dev = 0;
+  static std::atomic<int> sms[64];     // any host thread
+  int dev = 0, n = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return 0; }
-  if (sms[dev] == 0 &&
-      cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    cudaGetLastError();
-  return sms[dev];
+  n = sms[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    sms[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
 }
 
 bool rec_reg_supported(int T, int B, int d, int compact) {

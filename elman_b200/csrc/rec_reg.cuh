@@ -106,6 +106,12 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+// Elementwise functions in hardware precision, as in the TMEM kernels; widths and batches that came from the
+// CUDA-core kernel had tanhf and an IEEE division there.  Measured against 64 bits at those shapes: of 487 000
+// values of h none rounds to another bf16 number (|x| from 0.05 to 3 times a normal variate), of h silu(z) 6 in
+// 10^4 do (before: 1 in 10^5), its relative error is the same in five digits, and over whole sequences (200 x
+// 37 x 952 and others) no output or gradient is further off than summation order makes it.  With tanhf and
+// the division instead, 200 x 37 x 952 forward and backward takes 772 us instead of 703.
 __device__ __forceinline__ float tanh_fast(float x) {
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
