@@ -18,6 +18,7 @@ from elman_b200 import mamba_gated_elman as e1mod
 from elman_b200 import pure_lowrank_elman as e5mod
 from elman_b200 import stock_elman as e0mod
 from oracle import elman_oracle as orc
+from tests._gpu_cases import option
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-4
@@ -228,10 +229,18 @@ def test_e33_self_gate_bf16_tensor_core_path_matches_oracle(T, B, d):
         assert orc.rel_err(got[k].float().cpu(), w) < 2e-2, k
 
 
-@pytest.mark.parametrize("T,B,d,r", [(12, 16, 256, 64), (20, 32, 512, 100), (64, 32, 1536, 270)])
-def test_e4_lowrank_bf16_tensor_core_path_matches_oracle(T, B, d, r):
-    """E4 (dense W_x, low-rank recurrent matrix, z as gate input) on the single-cluster low-rank
-    kernel, every output and gradient against the fp32 oracle; rank 100 and 270 are zero-padded."""
+@pytest.fixture(params=[0, 1], ids=["registers", "cluster"])
+def either_kernel(request):
+    with option("rec_reg", request.param):
+        yield
+
+
+@pytest.mark.parametrize("T,B,d,r", [(12, 16, 256, 64), (20, 32, 512, 100), (64, 32, 1536, 270), (6, 40, 136, 20),
+                                     (5, 128, 1536, 270)])
+def test_e4_lowrank_bf16_tensor_core_path_matches_oracle(T, B, d, r, either_kernel):
+    """E4 (dense W_x, low-rank recurrent matrix, z as gate input) on the low-rank kernels, every output
+    and gradient against the fp32 oracle; rank 100 and 270 are zero-padded.  (The last two shapes: the rank
+    vector in two parts, or the CUDA cores.)"""
     from elman_b200 import hasty_pytorch_lib as H
     inp = orc.make_e1_inputs(T, B, d, seed=444 + d)
     g = torch.Generator().manual_seed(d + r)
